@@ -344,9 +344,11 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
         while (mz > 1 && !back_mz_fits(p, mz)) mz >>= 1;
         p->back_mz = p->back_mz_tf = mz;
         p->back_qcap = p->back_qcap_tf = back_qcap_for(p, mz);
-        // FDK: one z block of 32 voxels per lane measured fastest on B200 (config 2:
-        // 124 ms against 179 ms for eight)
-        p->pd_mz = 1;
+        // FDK: a pass of all slices up to 256, in pairs of 32-voxel blocks.  Measured on B200,
+        // back,hpd with 1, 2, 4 and 8 blocks: 512^2 x 256, 90 views 11.6, 7.7, 7.4 and 7.1 ms;
+        // 128^2 x 64, 360 views 0.79, 0.53, 0.60 and 0.60 ms (the longer kernels hold more
+        // registers); 211 x 187 x 93, 241 views 1.95, 1.66, 1.56 and 1.63 ms.
+        p->pd_mz = std::min(8, pow2_at_least((G.nz + 31) / 32));
     }
 
     // device allocations
@@ -477,6 +479,16 @@ extern "C" ctsim_status ctsim_plan_project(ctsim_plan *p, int method, const floa
                                            int view_begin, int view_stride, int view_count, void *stream) {
     return ctsim_plan_project_ex(p, method, d_image, CTSIM_F32, d_proj, CTSIM_F32, view_begin, view_stride,
                                  view_count, stream);
+}
+
+// back,hpd of all views of a sinogram in proj_dtype into the FP32 image, times scale, then
+// times scale2 (fdk.cu: dbeta and the change of units).
+ctsim_status ctsim_plan_back_hpd(ctsim_plan *p, const void *d_proj, int proj_dtype, float *d_image, float scale,
+                                 float scale2, cudaStream_t st) {
+    if (p->g.det == 2) return fail(CTSIM_ERR_UNSUPPORTED, kArcOnlyDD);
+    const cudaError_t e = launch_pd(kPdClamp, p->pd_mz, p->g, p->d_views, d_proj, p->d_map, d_image, CTSIM_F32, 0, 1,
+                                    p->geom.noviews, scale, st, false, proj_dtype, scale2);
+    return e == cudaSuccess ? CTSIM_OK : cuda_fail(e, "backprojection kernel");
 }
 
 extern "C" ctsim_status ctsim_plan_backproject_ex(ctsim_plan *p, int method, const void *d_proj, int proj_dtype,

@@ -21,6 +21,8 @@ extern ctsim_status ctsim_set_last_error(ctsim_status s, const char *msg);
 // plan internals shared with capi.cu
 extern const double *ctsim_plan_betas(const ctsim_plan *p);
 extern const ctsim_geom *ctsim_plan_geom(const ctsim_plan *p);
+extern ctsim_status ctsim_plan_back_hpd(ctsim_plan *p, const void *d_proj, int proj_dtype, float *d_image, float scale,
+                                        float scale2, cudaStream_t st);
 extern cudaError_t ctsim_plan_alloc(const ctsim_plan *p, void **ptr, size_t n);
 extern void ctsim_plan_release(const ctsim_plan *p, void *ptr);
 extern cudaError_t ctsim_plan_upload(const ctsim_plan *p, void *dst, const void *src, size_t n);
@@ -373,13 +375,7 @@ extern "C" ctsim_status ctsim_fdk_run_ex(ctsim_fdk *f, const void *d_sino, int s
     ctsim_status s = fdk_filter(f, d_sino, sino_dtype, f->d_filtered, sino_dtype, stream);
     if (s != CTSIM_OK) return s;
     // img = backProjectMex(sino, geom, 1, 0, 'back,hpd') * dbeta * 10  (reconFDK.m:84)
-    s = ctsim_plan_backproject_ex(f->plan, CTSIM_BACK_HPD, f->d_filtered, sino_dtype, d_image, kF32, 0, 1, f->nviews,
-                                  f->dbeta, stream);
-    if (s != CTSIM_OK) return s;
-    const ctsim_geom &G = *ctsim_plan_geom(f->plan);
-    cudaError_t e = launch_scale(d_image, (size_t)G.nx * G.ny * G.nz, 10.0f, (cudaStream_t)stream);
-    if (e != cudaSuccess) return ctsim_set_last_error(CTSIM_ERR_CUDA, cudaGetErrorString(e));
-    return CTSIM_OK;
+    return ctsim_plan_back_hpd(f->plan, f->d_filtered, sino_dtype, d_image, f->dbeta, 10.0f, (cudaStream_t)stream);
 }
 
 extern "C" ctsim_status ctsim_fdk_run(ctsim_fdk *f, const float *d_sino, float *d_image, void *stream) {

@@ -3,8 +3,8 @@
 //   back_kernel<METHOD,MZ>   matched backprojection A^T (distance-driven / separable footprint)
 //   prefix_kernel            per-column axial prefix sums of the volume (input of A)
 //   proj_kernel<METHOD>      forward projection A
-//   pd_kernel<OFF,MZ>        voxel-driven bilinear FDK backprojection (back,pd / back,hpd)
-//   scale_kernel             y *= s
+//
+// The voxel-driven FDK backprojection is in pd.cu.
 //
 // Layouts (reference MEX conventions): image[iz][iy][ix], proj[view][iu][iv].
 #include "kernels.cuh"
@@ -1114,156 +1114,6 @@ __global__ void __launch_bounds__(kProjMaxThreads, 3) proj_staged_kernel(Geom g,
 }
 
 // ---------------------------------------------------------------------------
-// FDK voxel-driven bilinear backprojection (geom/cbct/cbct_back.c:7-133): warp
-// per column, lanes along z.  Per-view column quantities (u, w2, w2s) are computed
-// by lane j for view k0+j and broadcast; every voxel accumulates the views in the
-// reference's order with its exact float operations.
-// ---------------------------------------------------------------------------
-// SUM: the FP32 image holds the view sum of earlier view chunks (scale 1), which the
-// kernel continues in the same view order (separate instantiations).
-// One sinogram sample of storage type DT (kF32, kBF16, kF16) as float (exact widening).
-template <int DT>
-__device__ __forceinline__ float ld_sino(const void *__restrict__ base, size_t i) {
-    if (DT == kBF16) return __uint_as_float((unsigned)__ldg(static_cast<const unsigned short *>(base) + i) << 16);
-    if (DT == kF16) return __half2float(__ushort_as_half(__ldg(static_cast<const unsigned short *>(base) + i)));
-    return __ldg(static_cast<const float *>(base) + i);
-}
-
-// DT: the sinogram's storage type, read as it is (widening to FP32 is exact, so the
-// result equals that of an FP32 copy bit for bit).
-template <int MODE, int MZ, bool SUM = false, int DT = kF32>
-__global__ void __launch_bounds__(256) pd_kernel(Geom g, const View *__restrict__ views,
-                                                 const void *__restrict__ proj, const uint8_t *__restrict__ map,
-                                                 void *__restrict__ image, int out_dtype, int view_begin,
-                                                 int view_stride, int view_count, float scale) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_x = (g.nx + 7) >> 3;
-    const int iy = blockIdx.x / tiles_x;
-    const int ix = (blockIdx.x % tiles_x) * 8 + warp;
-    if (ix >= g.nx || iy >= g.ny) return;
-    // per view of the current 32-view chunk, written by the view's own lane:
-    // {wul, omu, w2, w2s}, {couch, 1 if u is on the detector else 0, bits of the detector
-    // column's element offset}
-    __shared__ float4 vtab[8][32][2];
-    const size_t nxy = (size_t)g.nx * g.ny;
-    const size_t nuv = (size_t)g.nu * g.nv;
-    const bool on = map[iy * g.nx + ix] != 0;
-    const float xc = fmul(fadd((float)ix, g.wx), g.dx);
-    const float yc = fmul(fadd((float)iy, g.wy), g.dy);
-    const int zpass = 32 * MZ;
-    for (int iz0 = 0; iz0 < g.nz; iz0 += zpass) {
-        const int izn = min(zpass, g.nz - iz0);
-        float acc[MZ], zc0[MZ];
-#pragma unroll
-        for (int m = 0; m < MZ; m++) {
-            acc[m] = 0.0f;
-            zc0[m] = fmul(fadd((float)(iz0 + lane + 32 * m), g.wz_pd), g.dz);  // (iz + wz) * dz, cbct_back.c:100
-        }
-        if (SUM) {
-            const float *src = static_cast<const float *>(image) + (size_t)(iz0 + lane) * nxy + (size_t)iy * g.nx + ix;
-#pragma unroll
-            for (int m = 0; m < MZ; m++)
-                if (lane + 32 * m < izn) acc[m] = src[(size_t)(32 * m) * nxy];
-        }
-        if (on) {
-            for (int k0 = 0; k0 < view_count; k0 += 32) {
-                constexpr bool OFF = MODE != kPdClamp, VAR = MODE == kPdVar;
-                float u = -1.0f, w2 = 0.0f, w2s = 0.0f, couch = 0.0f;
-                const int kl = k0 + lane;
-                if (kl < view_count) {
-                    const View v = views[view_begin + kl * view_stride];
-                    const float xr = fsub(fmul(xc, v.cos_a), fmul(yc, v.sin_a));
-                    const float yr = fadd(fmul(xc, v.sin_a), fmul(yc, v.cos_a));
-                    const float den = fadd(g.sad, yr);
-                    if (g.det == 1) {  // cbct_back.c:68-77
-                        w2 = fdiv(g.sdd, den);
-                        w2s = fmul(w2, w2);
-                        u = fsub(fdiv(fmul(xr, w2), g.du), g.wu);
-                    } else {           // cbct_back.c:78-88, cbct_back_var.c:68-77
-                        const float xo = fsub(xr, VAR ? g.roff_var : g.roff);
-                        const double at = atan((double)fdiv(xo, den));
-                        u = (float)__dsub_rn(__ddiv_rn(__dmul_rn(at, (double)g.sdd), (double)g.du), (double)g.wu);
-                        w2s = fdiv(fmul(g.sdd, g.sdd), fadd(fmul(den, den), fmul(xo, xo)));
-                        w2 = fdiv(g.sdd, den);
-                    }
-                    couch = VAR ? v.wz : v.couch_pd;  // back,var: the couch shift is in wz
-                }
-                {
-                    // this lane's view: the detector column and u weights (cbct_back.c:90-99)
-                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = make_float4(couch, __int_as_float(0), 0.f, 0.f);
-                    if (kl < view_count && u >= g.u_lo && u <= g.u_hi) {  // cbct_back.c:90
-                        float fiu;
-                        const int iu = floor_pos(u, &fiu);
-                        const float wul = fsub(u, fiu);
-                        a = make_float4(wul, fsub(1.0f, wul), w2, w2s);
-                        const unsigned long long pv = (unsigned long long)kl * nuv + (unsigned long long)iu * g.nv;
-                        b.y = __int_as_float(1);
-                        b.z = __uint_as_float((unsigned)pv);
-                        b.w = __uint_as_float((unsigned)(pv >> 32));
-                    }
-                    __syncwarp();  // the previous chunk's reads are done
-                    vtab[warp][lane][0] = a;
-                    vtab[warp][lane][1] = b;
-                }
-                __syncwarp();
-                const int nk = min(32, view_count - k0);
-                for (int j = 0; j < nk; j++) {
-                    const float4 b = vtab[warp][j][1];
-                    if (__float_as_int(b.y) == 0) continue;  // u off the detector
-                    const float4 a = vtab[warp][j][0];
-                    const float wul = a.x, omu = a.y, w2j = a.z, w2sj = a.w, cj = b.x;
-                    const size_t pv = ((size_t)__float_as_uint(b.w) << 32) | __float_as_uint(b.z);  // element offset
-#pragma unroll
-                    for (int m = 0; m < MZ; m++) {
-                        if (lane + 32 * m < izn) {
-                            // (iz + wz) * dz + couch (cbct_back.c:100); back,var: (iz + wz) * dz with
-                            // the view's wz (cbct_back_var.c:41, :89)
-                            const float zc = VAR ? fmul(fadd((float)(iz0 + lane + 32 * m), cj), g.dz)
-                                                 : fadd(zc0[m], cj);
-                            float vv = fsub(div_by(fmul(zc, w2j), g.dv, g.rdv), g.wv);  // cbct_back.c:102
-                            bool use = true;
-                            if (OFF) {
-                                use = vv >= g.v_lo && vv <= g.v_hi;  // cbct_back.c:105-108
-                            } else {
-                                vv = vv > 0.5f ? vv : 0.5f;          // cbct_back.c:110-111
-                                vv = vv < g.v_clamp_hi ? vv : g.v_clamp_hi;
-                            }
-                            if (use) {
-                                float fiv;
-                                const int iv = min(floor_pos(vv, &fiv), g.nv - 2);
-                                const float wvl = fsub(vv, fiv);
-                                const float omv = fsub(1.0f, wvl);
-                                const size_t p = pv + iv;
-                                const float s0 = fadd(fmul(omv, ld_sino<DT>(proj, p)), fmul(wvl, ld_sino<DT>(proj, p + 1)));
-                                const float s1 = fadd(fmul(omv, ld_sino<DT>(proj, p + g.nv)),
-                                                      fmul(wvl, ld_sino<DT>(proj, p + g.nv + 1)));
-                                const float val = fadd(fmul(omu, s0), fmul(wul, s1));
-                                // w2s * (...) (cbct_back.c:120); w2s * w2s * (...) (cbct_back_var.c:116)
-                                acc[m] = fadd(acc[m], fmul(VAR ? fmul(w2sj, w2sj) : w2sj, val));
-                            }
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < MZ; m++) {
-            const int dz = lane + 32 * m;
-            if (dz < izn) {
-                float r = on ? acc[m] : 0.0f;
-                if (scale != 1.0f) r = r * scale;
-                store_from_float(image, (size_t)(iz0 + dz) * nxy + (size_t)iy * g.nx + ix, r, out_dtype);
-            }
-        }
-    }
-}
-
-__global__ void scale_kernel(float *__restrict__ y, size_t n, float s) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        y[i] *= s;
-}
-
-// ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
 // The dynamic shared-memory limit is a per-function, per-device attribute shared by
@@ -1443,47 +1293,6 @@ cudaError_t launch_proj(int method, int groups, int rows, bool pairs, const Geom
     CTSIM_PROJ_CASE(kTF, 4, true) CTSIM_PROJ_CASE(kTF, 8, true)
 #undef CTSIM_PROJ_CASE
     return cudaErrorInvalidValue;
-}
-
-template <int MODE, int MZ>
-static cudaError_t launch_pd_mz(const Geom &g, const View *views, const void *proj, int in_dtype, const uint8_t *map,
-                                void *image, int out_dtype, int vb, int vs, int vc, float scale, bool accumulate,
-                                cudaStream_t st) {
-    const int blocks = g.ny * ((g.nx + 7) / 8);
-    if (accumulate)
-        pd_kernel<MODE, MZ, true><<<blocks, 256, 0, st>>>(g, views, proj, map, image, out_dtype, vb, vs, vc, scale);
-    else if (in_dtype == kBF16)
-        pd_kernel<MODE, MZ, false, kBF16><<<blocks, 256, 0, st>>>(g, views, proj, map, image, out_dtype, vb, vs, vc,
-                                                                  scale);
-    else if (in_dtype == kF16)
-        pd_kernel<MODE, MZ, false, kF16><<<blocks, 256, 0, st>>>(g, views, proj, map, image, out_dtype, vb, vs, vc,
-                                                                 scale);
-    else
-        pd_kernel<MODE, MZ><<<blocks, 256, 0, st>>>(g, views, proj, map, image, out_dtype, vb, vs, vc, scale);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pd(int mode, int mz, const Geom &g, const View *views, const void *proj, const uint8_t *map,
-                      void *image, int out_dtype, int vb, int vs, int vc, float scale, cudaStream_t st,
-                      bool accumulate, int in_dtype) {
-    if (accumulate && (out_dtype != kF32 || scale != 1.0f || in_dtype != kF32)) return cudaErrorInvalidValue;
-    if (in_dtype != kF32 && in_dtype != kBF16 && in_dtype != kF16) return cudaErrorInvalidValue;
-#define CTSIM_PD_CASE(O, Z)                                                                                    \
-    if (mode == O && mz == Z)                                                                                  \
-        return launch_pd_mz<O, Z>(g, views, proj, in_dtype, map, image, out_dtype, vb, vs, vc, scale, accumulate, \
-                                  st);
-    CTSIM_PD_CASE(kPdOff, 1) CTSIM_PD_CASE(kPdOff, 2) CTSIM_PD_CASE(kPdOff, 4) CTSIM_PD_CASE(kPdOff, 8)
-    CTSIM_PD_CASE(kPdClamp, 1) CTSIM_PD_CASE(kPdClamp, 2) CTSIM_PD_CASE(kPdClamp, 4) CTSIM_PD_CASE(kPdClamp, 8)
-    CTSIM_PD_CASE(kPdVar, 1) CTSIM_PD_CASE(kPdVar, 2) CTSIM_PD_CASE(kPdVar, 4) CTSIM_PD_CASE(kPdVar, 8)
-#undef CTSIM_PD_CASE
-    return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_scale(float *y, size_t n, float s, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    scale_kernel<<<blocks, 256, 0, st>>>(y, n, s);
-    return cudaGetLastError();
 }
 
 // A^T reading the unscaled sinogram (axial amplitude applied on the fly); used by the

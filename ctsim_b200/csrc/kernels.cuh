@@ -56,12 +56,12 @@ bool proj_slots_valid(int xstride, int slots);
 // voxel-driven bilinear modes: back,pd (v outside the detector skipped), back,hpd (v
 // clamped), back,var (geom/cbct/cbct_back_var.c)
 enum PdMode { kPdOff = 0, kPdClamp = 1, kPdVar = 2 };
-// proj in storage type in_dtype (kF32, kBF16, kF16), read as it is.
+// proj in storage type in_dtype (kF32, kBF16, kF16), read as it is; the image is
+// (sum * scale) * scale2.
 cudaError_t launch_pd(int mode, int mz, const Geom &g, const View *views, const void *proj,
                       const uint8_t *map, void *image, int out_dtype, int view_begin, int view_stride,
-                      int view_count, float scale, cudaStream_t st, bool accumulate = false, int in_dtype = kF32);
-
-cudaError_t launch_scale(float *y, size_t n, float s, cudaStream_t st);
+                      int view_count, float scale, cudaStream_t st, bool accumulate = false, int in_dtype = kF32,
+                      float scale2 = 1.0f);
 
 // ---------------------------------------------------------------------------
 // Batched launches: the blocks of many plans' A (or A^T) in one persistent grid.
