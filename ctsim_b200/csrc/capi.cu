@@ -64,7 +64,7 @@ struct ctsim_plan {
     View *d_views = nullptr;
     float *d_ampv = nullptr;
     uint8_t *d_map = nullptr;
-    float *d_xs = nullptr;   // axial prefix sums [nx*ny][g.xstride] (or pairs [nx*ny][nz+1][2]) -- forward projector scratch
+    float *d_xs = nullptr;   // voxel columns or their prefix sums [nx*ny][g.xstride] (or pairs [nx*ny][nz+1][2]) -- forward scratch
     float *d_ps = nullptr;   // sinogram scaled by ampv [noviews][nu][nv] -- backprojector scratch
     int *d_err = nullptr;
     size_t bytes = 0;
@@ -72,11 +72,12 @@ struct ctsim_plan {
     float zinc_max = 0.f;    // upper bound of a voxel's height in detector rows
     int back_mz = 1, back_qcap = 0, pd_mz = 1;  // A^T (DD) and FDK z-pass depths (tunable)
     int back_mz_tf = 1, back_qcap_tf = 0;       // A^T (SF) z-pass depth (tunable)
-    int fwd_groups = 1;      // candidate groups of the forward projector (tunable)
-    int fwd_rows = 32;       // row threads per group of the forward projector (tunable)
-    bool fwd_pairs = false;  // prefix sums stored as (X, slope) pairs (small volumes; tunable)
-    bool fwd_staged = false; // plain sums, candidate columns staged in shared memory (tunable)
-    int fwd_slots = 8;       // prefix columns per stage buffer of the staged projector (tunable)
+    int fwd_groups = 1;      // candidate groups of the unstaged forward projector (tunable)
+    int fwd_sgroups = 1;     // candidate groups of the staged forward projector (tunable)
+    int fwd_rows = 32;       // row threads per group of the unstaged forward projector (tunable)
+    bool fwd_pairs = false;  // prefix sums stored as (X, slope) pairs (tunable)
+    bool fwd_staged = false; // voxel columns staged in shared memory (tunable)
+    int fwd_slots = 16;      // columns per stage buffer of the staged projector (tunable)
     bool xs_holds_pairs = false;  // the prefix scratch was sized for pairs
     bool fwd_ok = true;
     std::string fwd_reason;
@@ -227,7 +228,6 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     g.sdd_du = G.sdd / G.du;
     g.dz_dv = G.dz / G.dv;
     g.wz_pd = centre(G.nz, G.offset_z);
-    g.xstride = prefix_stride(G.nz);
     g.roff = G.offset_u * G.du * G.sad / G.sdd;
     g.roff_var = G.offset_u * G.sad / G.sdd;
     g.add = G.add;
@@ -302,6 +302,16 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
         return fail(CTSIM_ERR_UNSUPPORTED, "the source orbit must lie outside the volume (SAD > volume radius)");
     }
     p->zinc_max = (float)((double)G.dz / G.dv * G.sdd / ((double)G.sad - rmax) * 1.0001 + 1e-6);
+    {
+        // longest extent of a detector row in voxels (the farthest columns): `taps` voxels from
+        // the one its lower edge lies in, and the zeros below voxel 0 that an extent clamped
+        // there may cover
+        const double len = (double)G.dv / G.dz * ((double)G.sad + rmax) / G.sdd * 1.0001 + 1e-6;
+        const int whole = (int)std::min(std::floor(len), 1e6);
+        g.xpad = whole + 1;
+        g.taps = whole + 2;
+        g.xstride = column_stride(G.nz, g.xpad, g.taps);
+    }
     const double umm = std::max(std::fabs((double)g.wu * G.du), std::fabs(((double)G.nu - 1 + g.wu) * G.du)) + G.du;
     double stretch = G.detector_type == 1 ? 1.0 + (umm / G.sdd) * (umm / G.sdd) : 1.0;
     if (G.detector_type == 2) {
@@ -366,15 +376,20 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     CTSIM_ALLOC(p->d_ampv, sizeof(float) * ampv.size());
     CTSIM_ALLOC(p->d_map, mp.size());
     CTSIM_ALLOC(p->d_err, sizeof(int));
-    p->fwd_pairs = p->xs_holds_pairs = forward_pairs(nxy, G.nz);
-    // volumes whose prefix sums do not stay cache-resident: candidate columns staged in
-    // shared memory (B200, config 2: DD A 167 -> 146 ms)
-    p->fwd_slots = 8;
-    p->fwd_staged = !p->fwd_pairs && proj_slots_valid(g.xstride, p->fwd_slots) &&
-                    proj_staged_smem_bytes(G.nv, G.nx, G.ny, g.xstride, p->fwd_groups, p->fwd_rows, p->fwd_slots) <=
-                        200 * 1024;
+    p->xs_holds_pairs = forward_pairs(nxy, G.nz);
+    // the staged projector: as many columns per stage as leave room for two blocks on an SM
+    p->fwd_sgroups = 1;
+    auto staged_bytes = [&](int slots) {
+        return proj_staged_smem_bytes(G.nv, std::max(G.nx, G.ny), g.xstride, p->fwd_sgroups, slots);
+    };
+    p->fwd_slots = 32;
+    while (p->fwd_slots > 8 && staged_bytes(p->fwd_slots) > 110 * 1024) p->fwd_slots -= 8;
+    p->fwd_staged = (g.taps <= 3 || !p->xs_holds_pairs) && proj_slots_valid(g.xstride, p->fwd_slots) &&
+                    staged_bytes(p->fwd_slots) <= 200 * 1024;
+    p->fwd_pairs = p->xs_holds_pairs && !p->fwd_staged;
     if (p->fwd_ok)
-        CTSIM_ALLOC(p->d_xs, sizeof(float) * (size_t)nxy * (p->xs_holds_pairs ? 2 * (G.nz + 1) : g.xstride));
+        CTSIM_ALLOC(p->d_xs, sizeof(float) * (size_t)nxy *
+                                 std::max(g.xstride, p->xs_holds_pairs ? 2 * (G.nz + 1) : 0));
     // the backprojection scratch (an FP32 copy of the sinogram times ampv) is allocated on
     // first use (ensure_scratch): BF16/FP16 sinograms and CTSIM_INPUT_SCALED residuals are
     // read as they are and never need it
@@ -446,7 +461,15 @@ static ctsim_status ensure_scratch(ctsim_plan *p, cudaStream_t st) {
     return CTSIM_OK;
 }
 
-// prefix = false reuses the column prefix sums of the previous call on the same image
+// The image in the form the plan's forward projector reads: voxel columns (staged), or
+// column prefix sums.
+static cudaError_t prepare_image(const ctsim_plan *p, const void *d_image, int image_dtype, cudaStream_t st) {
+    const int nxy = p->g.nx * p->g.ny;
+    if (p->fwd_staged) return launch_columns(d_image, image_dtype, p->d_xs, nxy, p->g.nz, p->g.xpad, p->g.xstride, st);
+    return launch_prefix(d_image, image_dtype, p->d_xs, nxy, p->g.nz, p->fwd_pairs, p->g.xstride, st);
+}
+
+// prefix = false reuses the image form that the previous call on the same image left
 // (the host-pointer path projects one image in view chunks).
 static ctsim_status plan_project(ctsim_plan *p, int method, const void *d_image, int image_dtype, void *d_proj,
                                  int proj_dtype, int view_begin, int view_stride, int view_count, void *stream,
@@ -459,14 +482,12 @@ static ctsim_status plan_project(ctsim_plan *p, int method, const void *d_image,
     if (s != CTSIM_OK) return s;
     if (!p->fwd_ok) return fail(CTSIM_ERR_UNSUPPORTED, p->fwd_reason);
     cudaStream_t st = (cudaStream_t)stream;
-    const int nxy = p->g.nx * p->g.ny;
     cudaError_t e;
-    if (prefix && (e = launch_prefix(d_image, image_dtype, p->d_xs, nxy, p->g.nz, p->fwd_pairs, p->g.xstride, st)) != cudaSuccess)
-        return cuda_fail(e, "prefix kernel");
-    if (p->fwd_staged && !p->fwd_pairs)
-        e = launch_proj_staged(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_groups, p->fwd_rows, p->fwd_slots, p->g,
-                               p->d_views, p->d_xs, p->d_ampv, p->d_map, d_proj, proj_dtype, view_begin, view_stride,
-                               view_count, p->margin, p->d_err, st);
+    if (prefix && (e = prepare_image(p, d_image, image_dtype, st)) != cudaSuccess) return cuda_fail(e, "prefix kernel");
+    if (p->fwd_staged)
+        e = launch_proj_staged(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_sgroups, p->fwd_slots, p->g, p->d_views,
+                               p->d_xs, p->d_ampv, p->d_map, d_proj, proj_dtype, view_begin, view_stride, view_count,
+                               p->margin, p->d_err, st);
     else
         e = launch_proj(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_groups, p->fwd_rows, p->fwd_pairs, p->g,
                         p->d_views, p->d_xs, p->d_ampv, p->d_map, d_proj, proj_dtype, view_begin, view_stride,
@@ -542,13 +563,13 @@ extern "C" ctsim_status ctsim_plan_backproject_ex(ctsim_plan *p, int method, con
     return CTSIM_OK;
 }
 
-// Column prefix sums of an FP32 image for the forward projection of a later plan_project
-// with prefix = false.
+// The form of an FP32 image for the forward projection of a later plan_project with
+// prefix = false.
 static ctsim_status plan_prefix(ctsim_plan *p, int method, const void *d_image, cudaStream_t st) {
     if (method != CTSIM_PROJ_DD && method != CTSIM_PROJ_TF) return fail(CTSIM_ERR_ARGUMENT, "unknown forward method");
     if (p->g.det == 2 && method != CTSIM_PROJ_DD) return fail(CTSIM_ERR_UNSUPPORTED, kArcOnlyDD);
     if (!p->fwd_ok) return fail(CTSIM_ERR_UNSUPPORTED, p->fwd_reason);
-    const cudaError_t e = launch_prefix(d_image, CTSIM_F32, p->d_xs, p->g.nx * p->g.ny, p->g.nz, p->fwd_pairs, p->g.xstride, st);
+    const cudaError_t e = prepare_image(p, d_image, CTSIM_F32, st);
     return e == cudaSuccess ? CTSIM_OK : cuda_fail(e, "prefix kernel");
 }
 
@@ -1122,7 +1143,7 @@ extern "C" bool ctsim_cbct_geom(const char *type, CTSIM_GEOM_PARAMS, const float
 // ---------------------------------------------------------------------------
 extern "C" ctsim_status ctsim_plan_get_tuning(const ctsim_plan *p, ctsim_tuning *t) {
     if (!p || !t) return fail(CTSIM_ERR_ARGUMENT, "null argument");
-    t->proj_groups = p->fwd_groups;
+    t->proj_groups = p->fwd_staged ? p->fwd_sgroups : p->fwd_groups;
     t->proj_rows = p->fwd_rows;
     t->proj_layout = p->fwd_pairs ? 2 : p->fwd_staged ? 3 : 1;
     t->proj_slots = p->fwd_slots;
@@ -1150,18 +1171,17 @@ extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning 
     if (t->pd_mz && !mz_valid(t->pd_mz)) return fail(CTSIM_ERR_ARGUMENT, "pd_mz must be 1, 2, 4 or 8");
     if (t->proj_layout && t->proj_layout != 1 && t->proj_layout != 3 && !(t->proj_layout == 2 && p->xs_holds_pairs))
         return fail(CTSIM_ERR_ARGUMENT,
-                    "proj_layout must be 1 (sums), 2 (pairs, on a plan whose volume fits them) or 3 (staged sums)");
+                    "proj_layout must be 1 (sums), 2 (pairs, on a plan whose volume fits them) or 3 (staged columns)");
     {
-        const bool staged = t->proj_layout ? t->proj_layout == 3 : (p->fwd_staged && !p->fwd_pairs);
-        const int G = t->proj_groups ? t->proj_groups : p->fwd_groups;
-        const int R = t->proj_rows ? t->proj_rows : p->fwd_rows;
+        const bool staged = t->proj_layout ? t->proj_layout == 3 : p->fwd_staged;
+        const int G = t->proj_groups ? t->proj_groups : p->fwd_sgroups;
         const int S = t->proj_slots ? t->proj_slots : p->fwd_slots;
         if (t->proj_slots && !proj_slots_valid(p->g.xstride, t->proj_slots))
             return fail(CTSIM_ERR_ARGUMENT, "proj_slots must be 1 .. 64 with slots * column bytes < 1 MiB");
-        if (staged && proj_staged_smem_bytes(p->geom.nv, p->geom.nx, p->geom.ny, p->g.xstride, G, R, S) > 200 * 1024)
+        if (staged && proj_staged_smem_bytes(p->geom.nv, std::max(p->geom.nx, p->geom.ny), p->g.xstride, G, S) > 200 * 1024)
             return fail(CTSIM_ERR_ARGUMENT, "the staged forward projector's shared memory exceeds 200 KiB: fewer slots");
     }
-    if (t->proj_groups) p->fwd_groups = t->proj_groups;
+    if (t->proj_groups) p->fwd_groups = p->fwd_sgroups = t->proj_groups;
     if (t->proj_rows) p->fwd_rows = t->proj_rows;
     if (t->proj_slots) p->fwd_slots = t->proj_slots;
     if (t->proj_layout) {
@@ -1202,21 +1222,21 @@ static std::vector<ctsim_tuning> tuning_candidates(const ctsim_plan *p, int meth
         std::vector<int> rows = {rmax};
         if (rmax > 64) rows.push_back(64);
         if (rmax > 32) rows.push_back(32);
-        for (int R : rows) {
+        for (int R : rows)
             for (int Gr : {1, 2, 4, 8})
-                if (proj_shape_valid(G.nv, Gr, R) && proj_smem_bytes(G.nv, G.nx, G.ny, Gr, R) <= 200 * 1024) {
+                if (proj_shape_valid(G.nv, Gr, R) && proj_smem_bytes(G.nv, G.nx, G.ny, Gr, R) <= 200 * 1024)
                     for (int lay = p->xs_holds_pairs ? 2 : 1; lay >= 1; lay--) {
                         ctsim_tuning t = {Gr, 0, 0, 0, R, lay, 0};
                         out.push_back(t);
                     }
-                    for (int S : {8, 16, 32})
-                        if (proj_slots_valid(p->g.xstride, S) &&
-                            proj_staged_smem_bytes(G.nv, G.nx, G.ny, p->g.xstride, Gr, R, S) <= 200 * 1024) {
-                            ctsim_tuning t = {Gr, 0, 0, 0, R, 3, S};
-                            out.push_back(t);
-                        }
+        // staged (proj_rows does not matter to it: the smallest value is valid with every group count)
+        for (int Gr : {1, 2, 4, 8})
+            for (int S : {8, 16, 32})
+                if (proj_slots_valid(p->g.xstride, S) &&
+                    proj_staged_smem_bytes(G.nv, std::max(G.nx, G.ny), p->g.xstride, Gr, S) <= 200 * 1024) {
+                    ctsim_tuning t = {Gr, 0, 0, 0, 32, 3, S};
+                    out.push_back(t);
                 }
-        }
         return out;
     }
     for (int mz : {1, 2, 4, 8}) {
@@ -1345,29 +1365,33 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
     if (s != CTSIM_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
-    // column prefix sums of every image (each plan's own scratch)
-    for (int i = 0; i < n; i++) {
-        const ctsim_plan *p = items[i].plan;
-        if ((e = launch_prefix(items[i].in, items[i].in_dtype, p->d_xs, p->g.nx * p->g.ny, p->g.nz, p->fwd_pairs, p->g.xstride,
-                               st)) != cudaSuccess)
+    // every image in its plan's form (each plan's own scratch)
+    for (int i = 0; i < n; i++)
+        if ((e = prepare_image(items[i].plan, items[i].in, items[i].in_dtype, st)) != cudaSuccess)
             return cuda_fail(e, "prefix kernel");
-    }
-    // one persistent launch per launch-shape class (row threads, candidate groups, prefix
-    // layout: 0 plain, 1 pairs, 2 staged, with the staged slots)
-    std::map<std::vector<int>, std::vector<int>> classes;  // (row threads, groups, layout, FP32 out, slots)
+    // one persistent launch per launch-shape class: unstaged (0 plain or 1 pairs; row threads,
+    // groups, FP32 out) or staged (2; row pairs per warp, warps, groups, blocks along the
+    // rows, slots, taps, column stride)
+    const int m = method == CTSIM_PROJ_DD ? kDD : kTF;
+    std::map<std::vector<int>, std::vector<int>> classes;
     for (int i = 0; i < n; i++) {
         const ctsim_plan *p = items[i].plan;
-        const bool staged = p->fwd_staged && !p->fwd_pairs;
-        classes[{p->fwd_rows, p->fwd_groups, p->fwd_pairs ? 1 : staged ? 2 : 0,
-                 items[i].out_dtype == CTSIM_F32 ? 0 : 1, staged ? p->fwd_slots : 0}].push_back(i);
+        if (p->fwd_staged) {
+            const StagedShape S = staged_shape(p->geom.nv, p->fwd_sgroups);
+            classes[{2, S.np, S.warps, S.parts, S.groups, S.split, p->fwd_slots, p->g.taps, p->g.xstride}].push_back(i);
+        } else {
+            classes[{p->fwd_pairs ? 1 : 0, p->fwd_rows, p->fwd_groups, items[i].out_dtype == CTSIM_F32 ? 0 : 1}].push_back(i);
+        }
     }
     for (auto &cl : classes) {
-        const std::vector<int> &idx = cl.second;
+        const std::vector<int> &key = cl.first, &idx = cl.second;
+        const bool staged = key[0] == 2;
         for (size_t c0 = 0; c0 < idx.size(); c0 += kBatchMax) {
             ProjBatch b;
             b.n = 0;
             b.total = 0;
             size_t smem = 0;
+            int nlines = 1;
             for (size_t c = c0; c < std::min(idx.size(), c0 + kBatchMax); c++) {
                 const ctsim_batch_item &it = items[idx[c]];
                 const ctsim_plan *p = it.plan;
@@ -1382,22 +1406,20 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
                 T.vb = it.view_begin;
                 T.vs = it.view_stride;
                 T.vc = it.view_count;
-                T.gx = (p->g.nu + proj_group_width() - 1) / proj_group_width();
+                T.gx = staged ? staged_columns(StagedShape{key[1], key[2], key[3], key[4], key[5]}, p->g.nu)
+                              : (p->g.nu + kProjGroupWidth - 1) / kProjGroupWidth;
                 T.first = b.total;
                 T.margin = p->margin;
                 T.err = p->d_err;
-                b.total += proj_task_blocks(p->g, it.view_count);
-                smem = std::max(smem, cl.first[2] == 2 ? proj_staged_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->g.xstride,
-                                                                                p->fwd_groups, p->fwd_rows,
-                                                                                p->fwd_slots)
-                                                       : proj_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->fwd_groups,
-                                                                         p->fwd_rows));
+                b.total += T.gx * it.view_count * (staged ? key[5] : 1);
+                nlines = std::max(nlines, std::max(p->g.nx, p->g.ny));
+                smem = std::max(smem, staged ? proj_staged_smem_bytes(p->g.nv, nlines, p->g.xstride, p->fwd_sgroups,
+                                                                      p->fwd_slots)
+                                             : proj_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->fwd_groups, p->fwd_rows));
             }
-            const int m = method == CTSIM_PROJ_DD ? kDD : kTF;
-            e = cl.first[2] == 2 ? launch_proj_staged_batch(m, cl.first[1], cl.first[0], cl.first[4], cl.first[3] != 0,
-                                                            smem, b, st)
-                                 : launch_proj_batch(m, cl.first[1], cl.first[0], cl.first[2] == 1, cl.first[3] != 0,
-                                                     smem, b, st);
+            e = staged ? launch_proj_staged_batch(m, StagedShape{key[1], key[2], key[3], key[4], key[5]}, key[7], key[6], nlines, smem,
+                                                  b, st)
+                       : launch_proj_batch(m, key[2], key[1], key[0] == 1, key[3] != 0, smem, b, st);
             if (e != cudaSuccess) return cuda_fail(e, "batched forward projection");
         }
     }

@@ -53,13 +53,14 @@ struct Geom {
     float v_clamp_lo, v_clamp_hi; // hpd clamps 0.5 and nv - 1.5 as floats (cbct_back.c:110-111)
     float rdv;                    // RN(1/dv) for the correctly rounded division by dv, 0 = use IEEE division
     float add, sad_add;           // arc detector: radius ADD, sad / add (geom/cbct/cbct_proj3.c:337-355)
-    int xstride;                  // column stride (floats) of the plain prefix-sum layout: prefix_stride(nz)
+    int xstride;                  // column stride (floats) of the plain prefix sums and of the staged columns
+    int xpad, taps;               // staged columns: zeros below voxel 0; voxels that a detector row can reach
 };
 
-// Column stride of the plain prefix-sum layout: X[0..nz] and at least one copy of X[nz]
-// above it, rounded up to 4 floats so that every column starts on a 16-byte boundary
-// (the bulk copies of the staged forward projector need that).
-__host__ __device__ inline int prefix_stride(int nz) { return (nz + 2 + 3) & ~3; }
+// Column stride of the plain prefix sums (X[0..nz] and X[nz] repeated above it) and of the
+// staged columns (xpad zeros, nz voxels, `taps` zeros), rounded up to 4 floats so that every
+// column starts on a 16-byte boundary (the bulk copies need that).  xpad >= 1, taps >= 2.
+__host__ __device__ inline int column_stride(int nz, int xpad, int taps) { return (nz + xpad + taps + 3) & ~3; }
 
 // Per-view constants, geom/cbct/cbct_proj.c:256-265 and cbct_back.c:50-52.
 struct View {
@@ -125,8 +126,9 @@ __device__ __forceinline__ float u_of(const Geom &g, float num, float den) {
 }
 
 // Exact transcription of the per-column footprint (DD: cbct_proj.c:282-372,
-// TF: cbct_proj.c:531-656).
-template <int METHOD>
+// TF: cbct_proj.c:531-656).  ROWS = false leaves the test out whether any of the column's
+// rows meets the detector (hit: its detector columns do).
+template <int METHOD, bool ROWS = true>
 __device__ __forceinline__ ColumnFP column_footprint(const Geom &g, const View &v, int ix, int iy) {
     ColumnFP c;
     c.hit = false;
@@ -187,6 +189,8 @@ __device__ __forceinline__ ColumnFP column_footprint(const Geom &g, const View &
     // axial footprint, cbct_proj.c:361-372
     c.zinc = fdiv(fmul(g.dz_dv, g.sdd), dsxy0);
     c.vstart = (float)__dsub_rn(__dmul_rn(__dsub_rn((double)v.wz, 0.5), (double)c.zinc), (double)g.wv);
+    c.hit = true;
+    if (!ROWS) return c;
     int s = (int)floorf(fdiv(fsub(-1.0f, c.vstart), c.zinc));
     int e = (int)ceilf(fdiv(fsub((float)(g.nv + 1), c.vstart), c.zinc));
     s = max(s, 0);

@@ -10,6 +10,24 @@
 
 namespace ctsim {
 
+// Detector columns per block of the forward projector.
+constexpr int kProjGroupWidth = 8;
+
+// Views per group of the forward projector's launch order.
+constexpr int kViewGroup = 32;
+
+// Detector-column group bx and launch view by of the forward projector's linear block
+// L: the launch views in groups of kViewGroup consecutive ones (the last group may be
+// shorter), and within a group the blocks of one detector-column group over all its
+// views, then the next column group -- neighbouring views share candidate columns in L2.
+__device__ __forceinline__ void view_grouped_block(int L, int ngx, int vc, int &bx, int &by) {
+    const int per = ngx * kViewGroup;
+    const int G = L / per, r = L - G * per;
+    const int n = min(kViewGroup, vc - G * kViewGroup);  // views of this group
+    bx = r / n;
+    by = G * kViewGroup + (r - bx * n);
+}
+
 // ps = proj (any storage type) * ampv (ampv may be null: plain conversion to FP32)
 cudaError_t launch_prescale(const void *proj, int in_dtype, const float *ampv, float *ps, size_t nuv, size_t n,
                             cudaStream_t st);
@@ -42,16 +60,24 @@ int proj_default_rows(int nv);
 bool proj_groups_valid(int nv, int groups);
 bool proj_shape_valid(int nv, int groups, int rows);
 size_t proj_smem_bytes(int nv, int nx, int ny, int groups, int rows);
-// The forward projector with each candidate's prefix column staged in shared memory by
-// bulk copies (plain layout, g.xstride a multiple of 4 and >= nz + 2, xs 16-byte aligned):
-// `slots` columns per stage buffer, two buffers.  A stage wait that runs out sets bit 4
-// of *err.
-cudaError_t launch_proj_staged(int method, int groups, int rows, int slots, const Geom &g, const View *views,
-                               const float *xs, const float *ampv, const uint8_t *map, void *proj, int out_dtype,
-                               int view_begin, int view_stride, int view_count, float margin, int *err,
-                               cudaStream_t st);
-size_t proj_staged_smem_bytes(int nv, int nx, int ny, int xstride, int groups, int rows, int slots);
+// The forward projector with the candidates' voxel columns staged in shared memory
+// (proj_staged.cu): xs holds the image as columns (launch_columns; 16-byte aligned),
+// up to `slots` of them per stage; candidate groups 1, 2, 4 or 8.  A stage wait
+// that runs out sets bit 4 of *err.
+cudaError_t launch_columns(const void *image, int in_dtype, float *xs, int nxy, int nz, int xpad, int xstride,
+                           cudaStream_t st);
+cudaError_t launch_proj_staged(int method, int groups, int slots, const Geom &g, const View *views, const float *xs,
+                               const float *ampv, const uint8_t *map, void *proj, int out_dtype, int view_begin,
+                               int view_stride, int view_count, float margin, int *err, cudaStream_t st);
+size_t proj_staged_smem_bytes(int nv, int nlines, int xstride, int groups, int slots);
 bool proj_slots_valid(int xstride, int slots);
+// Row pairs per consumer warp; consumer warps along the rows, the columns and the
+// candidates; blocks along the rows.
+struct StagedShape {
+    int np, warps, parts, groups, split;
+};
+StagedShape staged_shape(int nv, int groups);
+int staged_columns(const StagedShape &shape, int nu);
 
 // voxel-driven bilinear modes: back,pd (v outside the detector skipped), back,hpd (v
 // clamped), back,var (geom/cbct/cbct_back_var.c)
@@ -102,8 +128,7 @@ struct BackBatch {
     BackTask t[kBatchMax];
 };
 
-// The flat blocks of a task: A (u groups x views), A^T (rows x column tiles).
-int proj_task_blocks(const Geom &g, int view_count);
+// The flat blocks of an A^T task (rows x column tiles).
 int back_task_blocks(const Geom &g);
 int proj_row_threads_of(int nv);
 // lowp: some task stores BF16/FP16 (each task's out_dtype); otherwise all store FP32
@@ -111,15 +136,17 @@ cudaError_t launch_proj_batch(int method, int groups, int row_threads, bool pair
                               const ProjBatch &b, cudaStream_t st);
 cudaError_t launch_back_batch(int method, int mz, bool vec, bool lowp, size_t smem, const BackBatch &b,
                               cudaStream_t st, int src = kSrcScaled);
-// The staged forward projector (launch_proj_staged) over a batch of plain-layout plans.
-cudaError_t launch_proj_staged_batch(int method, int groups, int row_threads, int slots, bool lowp, size_t smem,
+// The staged forward projector (launch_proj_staged) over a batch of plans of one shape and
+// column stride; nlines: the largest max(nx, ny).
+cudaError_t launch_proj_staged_batch(int method, const StagedShape &shape, int taps, int slots, int nlines, size_t smem,
                                      const ProjBatch &b, cudaStream_t st);
+// Blocks of a persistent launch: the resident blocks of the device, at most `total`.
+int persistent_grid(const void *kernel, int threads, size_t smem, int total);
 
 // Raises (never lowers) a kernel's dynamic shared-memory limit on the current device.
 cudaError_t allow_dynamic_smem(const void *kfn, size_t bytes);
 
 size_t proj_smem_bytes(int nv, int nx, int ny, int groups);
-int proj_group_width();
 int proj_max_lines();
 
 }  // namespace ctsim

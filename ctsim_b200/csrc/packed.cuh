@@ -11,18 +11,14 @@
 
 namespace ctsim {
 
-struct f32x2 {
-    unsigned long long v;
-};
+using f32x2 = float2;
 
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-    return r;
-}
+__device__ __forceinline__ f32x2 pack2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ void unpack2(f32x2 x, float &a, float &b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+    a = x.x;
+    b = x.y;
 }
+
 // The same operations on one value (float) and on two (f32x2), so that a kernel body can
 // be written once for both widths.  All of them are round-to-nearest and never contracted,
 // except padd_rd (toward -inf) -- but see padd_product.
@@ -32,22 +28,13 @@ __device__ __forceinline__ float pmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float pfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float padd_rd(float a, float b) { return __fadd_rd(a, b); }
 
-#define CTSIM_PACKED_OP2(NAME, OP)                                                        \
-    __device__ __forceinline__ f32x2 NAME(f32x2 a, f32x2 b) {                             \
-        f32x2 r;                                                                          \
-        asm(OP " %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));                          \
-        return r;                                                                         \
-    }
-CTSIM_PACKED_OP2(padd, "add.rn.f32x2")
-CTSIM_PACKED_OP2(psub, "sub.rn.f32x2")
-CTSIM_PACKED_OP2(pmul, "mul.rn.f32x2")
-CTSIM_PACKED_OP2(padd_rd, "add.rm.f32x2")
-#undef CTSIM_PACKED_OP2
-__device__ __forceinline__ f32x2 pfma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
+__device__ __forceinline__ f32x2 padd(f32x2 a, f32x2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ f32x2 psub(f32x2 a, f32x2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ f32x2 pmul(f32x2 a, f32x2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ f32x2 padd_rd(f32x2 a, f32x2 b) { return __fadd2_rd(a, b); }
+__device__ __forceinline__ f32x2 pfma(f32x2 a, f32x2 b, f32x2 c) { return __ffma2_rn(a, b, c); }
+// a * b + c rounded toward -inf
+__device__ __forceinline__ f32x2 pfma_rd(f32x2 a, f32x2 b, f32x2 c) { return __ffma2_rd(a, b, c); }
 
 // x + y where x or y is a product that the reference rounds before it adds.  ptxas
 // contracts a packed product and a packed sum into one fma although both are marked .rn
@@ -73,11 +60,7 @@ template <>
 struct Packed<f32x2> {
     static constexpr int kWidth = 2;
     static __device__ __forceinline__ f32x2 all(float a) { return pack2(a, a); }
-    static __device__ __forceinline__ float get(f32x2 x, int i) {
-        float a, b;
-        unpack2(x, a, b);
-        return i ? b : a;
-    }
+    static __device__ __forceinline__ float get(f32x2 x, int i) { return i ? x.y : x.x; }
     template <class F>
     static __device__ __forceinline__ f32x2 make(F f) {
         const float a = f(0), b = f(1);
