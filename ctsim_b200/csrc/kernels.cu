@@ -1,10 +1,10 @@
 // Projector kernels for sm_100a.
 //
-//   back_kernel<METHOD,MZ>   matched backprojection A^T (distance-driven / separable footprint)
 //   prefix_kernel            per-column axial prefix sums of the volume (input of A)
 //   proj_kernel<METHOD>      forward projection A
 //
-// The voxel-driven FDK backprojection is in pd.cu.
+// The staged forward projector is in proj_staged.cu, the matched backprojection in back.cu,
+// the voxel-driven FDK backprojection in pd.cu.
 //
 // Layouts (reference MEX conventions): image[iz][iy][ix], proj[view][iu][iv].
 #include "kernels.cuh"
@@ -17,299 +17,8 @@ namespace ctsim {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// Rows r0 .. r0+3 of one detector column of a sinogram source (element offset off of row
-// r0), times ampv at the same element for the unscaled sources.  VEC: nv a multiple of 4
-// and the source aligned (one 16-byte FP32 or 8-byte 16-bit load); otherwise rows at or
-// past nv read as 0.
-template <int SRC, bool VEC>
-__device__ __forceinline__ float4 load_rows4(const void *__restrict__ src, const float *__restrict__ ampv, size_t off,
-                                             size_t aoff, int r0, int nv) {
-    float4 p;
-    if (SRC == kSrcScaled || SRC == kSrcF32) {
-        const float *pr = static_cast<const float *>(src) + off;
-        if (VEC) {
-            p = __ldg(reinterpret_cast<const float4 *>(pr));
-        } else {
-            p.x = __ldg(pr);
-            p.y = r0 + 1 < nv ? __ldg(pr + 1) : 0.f;
-            p.z = r0 + 2 < nv ? __ldg(pr + 2) : 0.f;
-            p.w = r0 + 3 < nv ? __ldg(pr + 3) : 0.f;
-        }
-    } else {
-        const unsigned short *pr = static_cast<const unsigned short *>(src) + off;
-        unsigned short h[4];
-        if (VEC) {
-            const uint2 u = __ldg(reinterpret_cast<const uint2 *>(pr));
-            h[0] = (unsigned short)(u.x & 0xffffu); h[1] = (unsigned short)(u.x >> 16);
-            h[2] = (unsigned short)(u.y & 0xffffu); h[3] = (unsigned short)(u.y >> 16);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; i++) h[i] = r0 + i < nv ? __ldg(pr + i) : (unsigned short)0;
-        }
-        float f[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            f[i] = SRC == kSrcBF16 ? __uint_as_float((unsigned)h[i] << 16) : __half2float(__ushort_as_half(h[i]));
-        p = make_float4(f[0], f[1], f[2], f[3]);
-    }
-    if (SRC != kSrcScaled) {  // axial amplitude applied here instead of in a scratch copy
-        const float *ar = ampv + aoff;
-        float4 a;
-        if (VEC) {
-            a = __ldg(reinterpret_cast<const float4 *>(ar));
-        } else {
-            a.x = __ldg(ar);
-            a.y = r0 + 1 < nv ? __ldg(ar + 1) : 0.f;
-            a.z = r0 + 2 < nv ? __ldg(ar + 2) : 0.f;
-            a.w = r0 + 3 < nv ? __ldg(ar + 3) : 0.f;
-        }
-        p.x *= a.x; p.y *= a.y; p.z *= a.z; p.w *= a.w;
-    }
-    return p;
-}
-
-// ---------------------------------------------------------------------------
-// A^T: one warp per voxel column, lanes along z; 8 columns (consecutive ix) per block.
-// For each view the warp forms, in shared memory, the u-weighted detector column
-//     q[iv] = sum_iu w_u(iu) * ps[iu][iv]        (ps = proj * ampv)
-// over the rows the column's voxels can touch (4 rows per lane, float4 loads).  Each
-// voxel then sums q over the rows its axial extent covers with the distance-driven
-// row weights of geom/cbct/cbct_back.c:318-357, its edges vmin/vmax computed with the
-// reference's float operations (usually two or three rows per voxel).  The edges sit
-// hundreds of rows up the detector, where one float rounding moves a voxel's weight by
-// ~1e-5 of itself; evaluating them exactly as the reference does keeps each voxel's
-// value within a few float roundings of the reference's instead of adding noise of
-// that size.  Accumulation over views stays in registers; no atomics.
-// ---------------------------------------------------------------------------
-// The work of one block (8 columns of one row iy), as a device function: the plain
-// kernel runs it for blockIdx.x, the batched kernel for each of its work items.
-// 32-bit shared load ordered after the warp's earlier shared stores (compiler barrier).
-__device__ __forceinline__ float lds_ordered(uint32_t a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-
-template <int METHOD, int MZ, bool VEC, int SRC, bool SUM = false>
-__device__ __forceinline__ void back_block(const Geom g, const View *__restrict__ views, const void *__restrict__ ps,
-                                           const uint8_t *__restrict__ map, void *__restrict__ image, int out_dtype,
-                                           int view_begin, int view_stride, int view_count, float scale, int qcap,
-                                           int *__restrict__ err, const float *__restrict__ ampv, float *smem,
-                                           int block) {
-    constexpr int kWS = 17;  // row stride of the per-warp weight table (conflict-free writes)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *wtab = smem + warp * (32 * kWS + 32 * 8 + qcap);  // [32 views][17] u weights of the view chunk
-    // [32 views] per-view scalars of the chunk, written by the view's own lane:
-    // {ampu, zinc, vstart, iumin | nb << 16}, {rbase | r_hi << 16, path + 1 (0: no rows), -, -}
-    float4 *vtab = reinterpret_cast<float4 *>(wtab + 32 * kWS);  // 16-byte aligned: 32 * 17 * 4 = 2176
-    float *Q = wtab + 32 * kWS + 32 * 8;                         // [qcap] q per row
-    const int tiles_x = (g.nx + 7) >> 3;
-    const int iy = block / tiles_x;
-    const int ix = (block % tiles_x) * 8 + warp;
-    if (ix >= g.nx || iy >= g.ny) return;
-    const size_t nxy = (size_t)g.nx * g.ny;
-    const size_t nuv = (size_t)g.nu * g.nv;
-    const bool on = map[iy * g.nx + ix] != 0;
-    const float fnv = (float)g.nv;
-    const int nvm1 = g.nv - 1;
-    const int zpass = 32 * MZ;
-    for (int iz0 = 0; iz0 < g.nz; iz0 += zpass) {
-        const int izn = min(zpass, g.nz - iz0);
-        const float fz_first = (float)iz0, fz_last = (float)(iz0 + izn - 1);
-        float acc[MZ];
-#pragma unroll
-        for (int m = 0; m < MZ; m++) acc[m] = 0.0f;
-        const float fz_lane = (float)(iz0 + lane);
-        if (SUM) {
-            // continue the per-voxel view sum (scale 1) that the previous view chunk left in
-            // the FP32 image; the sum runs in view order either way
-            const float *src = static_cast<const float *>(image) + (size_t)(iz0 + lane) * nxy + (size_t)iy * g.nx + ix;
-#pragma unroll
-            for (int m = 0; m < MZ; m++)
-                if (lane + 32 * m < izn) acc[m] = src[(size_t)(32 * m) * nxy];
-        }
-        if (on) {
-            for (int k0 = 0; k0 < view_count; k0 += 32) {
-                ColumnFP my;
-                my.hit = false;
-                const int kl = k0 + lane;
-                if (kl < view_count) my = column_footprint<METHOD>(g, views[view_begin + kl * view_stride], ix, iy);
-                // lane-parallel u weights of this lane's view (geom/cbct/cbct_back.c:288-301, :549-578)
-                // A voxel's vmax - vmin is zinc within 1.5 float ulps of nv (< 2^-10 for nv <=
-                // 8192), so away from zinc = 1 and 2 by a margin every voxel of the view covers
-                // the same number of rows give or take one: n = k_hi - k_lo is 0 or 1 (zinc < 1)
-                // or 1 or 2 (1 < zinc < 2).  Those views run branch-free (paths 1 and 2 below).
-                constexpr float kMargin = 1.0f / 256.0f;
-                __syncwarp();  // the previous chunk's reads of wtab and vtab are done
-                {
-                    int path1 = 0, rows = 0;
-                    if (my.hit) {
-                        const int nb = my.iumax - my.iumin + 1;
-                        for (int b = 0; b < nb; b++)
-                            wtab[lane * kWS + b] =
-                                u_weight<METHOD>(my.iumin + b, my.iumin, my.iumax, my.p0, my.p1, my.p2, my.p3);
-                        // rows reachable by voxels [iz0, iz0+izn) (the reference's clamped
-                        // extents, monotone in iz)
-                        const float zinc = my.zinc, vstart = my.vstart;
-                        const float a0u = fadd(fadd(vstart, fmul(fz_first, zinc)), 0.5f);
-                        const float b1u = fadd(fadd(fadd(vstart, fmul(fz_last, zinc)), zinc), 0.5f);
-                        const float a0 = fmaxf(a0u, 0.0f), b1 = fminf(b1u, fnv);
-                        if (a0 < fnv && b1 >= 0.0f) {
-                            const int r_lo = floor_pos(a0);
-                            int r_hi = min(floor_pos(b1), nvm1);
-                            if (r_lo <= r_hi) {
-                                const int rbase = r_lo & ~3;
-                                // every voxel of the pass exists and lies inside the detector
-                                bool inside = a0u > 0.0f && b1u < fnv && izn == zpass;
-                                if (r_hi - rbase + 1 > qcap) {  // rows rbase..r_hi must fit
-                                    atomicOr(err, 1);
-                                    r_hi = rbase + qcap - 1;
-                                    inside = false;
-                                }
-                                path1 = 1 + (!inside ? 0 : zinc < 1.0f - kMargin ? 1
-                                                     : (zinc > 1.0f + kMargin && zinc < 2.0f - kMargin) ? 2 : 0);
-                                rows = rbase | (r_hi << 16);
-                            }
-                        }
-                        vtab[2 * lane] = make_float4(my.ampu, zinc, vstart, __int_as_float(my.iumin | (nb << 16)));
-                    }
-                    vtab[2 * lane + 1] = make_float4(__int_as_float(rows), __int_as_float(path1), 0.f, 0.f);
-                }
-                __syncwarp();
-                const int nk = min(32, view_count - k0);
-                for (int j = 0; j < nk; j++) {
-                    const float4 pb = vtab[2 * j + 1];
-                    const int path1 = __float_as_int(pb.y);
-                    if (path1 == 0) continue;  // no footprint or no rows
-                    const float4 pa = vtab[2 * j];
-                    const float ampu = pa.x, zinc = pa.y, vstart = pa.z;
-                    const int iumin = __float_as_int(pa.w) & 0xffff, nb = __float_as_int(pa.w) >> 16;
-                    const int rbase = __float_as_int(pb.x) & 0xffff, r_hi = __float_as_int(pb.x) >> 16;
-                    // q over rows [rbase, r_hi], 128 rows per pass (the voxels read rows
-                    // [r_lo, r_hi] only)
-                    const float *wj = wtab + j * kWS;
-                    const size_t pv = (size_t)(k0 + j) * nuv + (size_t)iumin * g.nv;  // element offsets
-                    const size_t av = (size_t)iumin * g.nv;
-                    for (int c = rbase; c <= r_hi; c += 128) {
-                        const int r0 = c + 4 * lane;
-                        float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
-                        if (r0 <= r_hi) {
-                            for (int b = 0; b < nb; b++) {
-                                const float w = wj[b];
-                                const float4 p = load_rows4<SRC, VEC>(ps, ampv, pv + (size_t)b * g.nv + r0,
-                                                                      av + (size_t)b * g.nv + r0, r0, g.nv);
-                                q0 = fmaf(w, p.x, q0); q1 = fmaf(w, p.y, q1);
-                                q2 = fmaf(w, p.z, q2); q3 = fmaf(w, p.w, q3);
-                            }
-                        }
-                        *reinterpret_cast<float4 *>(Q + (r0 - rbase)) = make_float4(q0, q1, q2, q3);
-                    }
-                    __syncwarp();
-                    // Each voxel: the reference's clamped extent and row weights
-                    // (geom/cbct/cbct_back.c:318-357); rows [k_lo, k_hi] lie in [r_lo, r_hi]
-                    // because the edges are monotone in iz.
-                    const float *qb = Q - rbase;
-                    // shared address of row k is qadj + 4 * bits(k + 2^23) (mod 2^32)
-                    const uint32_t qadj = (uint32_t)__cvta_generic_to_shared(Q) - 4u * (uint32_t)rbase -
-                                          (0x4B000000u << 2);
-                    // Paths 1 and 2 always read the rows k_lo .. k_lo + 1 (+ 2) (the row buffer has 4
-                    // spare floats; rows past r_hi may hold anything, so their terms are selected,
-                    // never multiplied by zero).
-                    const int path = path1 - 1;
-                    if (path == 1) {
-#pragma unroll
-                        for (int m = 0; m < MZ; m++) {
-                            const float izv = fz_lane + (float)(32 * m);  // exact
-                            const float vpre = fadd(vstart, fmul(izv, zinc));
-                            const float vmin = fadd(vpre, 0.5f);
-                            const float vmax = fadd(fadd(vpre, zinc), 0.5f);
-                            const float tlo = __fadd_rd(vmin, kTwo23), thi = __fadd_rd(vmax, kTwo23);
-                            const uint32_t qa = qadj + (__float_as_uint(tlo) << 2);
-                            const float q0 = lds_ordered(qa), q1 = lds_ordered(qa + 4u);
-                            // one row: (vmax - vmin) q0; two: (k_lo + 1 - vmin) q0 + (vmax - k_hi) q1,
-                            // where k_hi = k_lo + 1 (kf, exact)
-                            const float one = fsub(vmax, vmin) * q0;
-                            const float kf = fsub(tlo, kTwo23 - 1.0f);
-                            const float two = fmaf(fsub(vmax, kf), q1, fsub(kf, vmin) * q0);
-                            acc[m] = fmaf(ampu, thi == tlo ? one : two, acc[m]);
-                        }
-                    } else if (path == 2) {
-#pragma unroll
-                        for (int m = 0; m < MZ; m++) {
-                            const float izv = fz_lane + (float)(32 * m);
-                            const float vpre = fadd(vstart, fmul(izv, zinc));
-                            const float vmin = fadd(vpre, 0.5f);
-                            const float vmax = fadd(fadd(vpre, zinc), 0.5f);
-                            const float tlo = __fadd_rd(vmin, kTwo23), thi = __fadd_rd(vmax, kTwo23);
-                            const uint32_t qa = qadj + (__float_as_uint(tlo) << 2);
-                            const float q0 = lds_ordered(qa), q1 = lds_ordered(qa + 4u), q2 = lds_ordered(qa + 8u);
-                            const bool three = fsub(thi, tlo) == 2.0f;
-                            const float wl = fsub(vmax, fsub(thi, kTwo23));
-                            // two rows: w0 q0 + wl q1; three: w0 q0 + q1 + wl q2 (the reference's row order)
-                            float vox = fmaf(three ? 1.0f : wl, q1, fsub(fsub(tlo, kTwo23 - 1.0f), vmin) * q0);
-                            vox = three ? fmaf(wl, q2, vox) : vox;
-                            acc[m] = fmaf(ampu, vox, acc[m]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int m = 0; m < MZ; m++) {
-                            const float izv = fz_lane + (float)(32 * m);  // exact
-                            const float vpre = fadd(vstart, fmul(izv, zinc));                // vstart + iz * zinc
-                            const float vmin = fmaxf(fadd(vpre, 0.5f), 0.0f);                 // max(vmin + 0.5, 0)
-                            const float vmax = fminf(fadd(fadd(vpre, zinc), 0.5f), fnv);      // min(vmax + 0.5, nv)
-                            if (izv <= fz_last && vmin <= vmax) {
-                                float flo, fhi;
-                                const int klo = floor_pos(vmin, &flo);
-                                int khi = floor_pos(vmax, &fhi);
-                                if (khi > nvm1) { khi = nvm1; fhi = fsub(fnv, 1.0f); }
-                                if (khi > klo + (kMaxRowsV - 1)) {
-                                    khi = klo + (kMaxRowsV - 1);
-                                    fhi = fadd(flo, (float)(kMaxRowsV - 1));
-                                }
-                                khi = min(khi, r_hi);  // only after a row-buffer overflow (flagged above)
-                                float vox = 0.0f;
-                                if (klo == khi) {
-                                    vox = fsub(vmax, vmin) * qb[klo];
-                                } else if (klo < khi) {
-                                    vox = fsub(fadd(flo, 1.0f), vmin) * qb[klo];
-                                    for (int k = klo + 1; k < khi; k++) vox += qb[k];
-                                    vox = fmaf(fsub(vmax, fhi), qb[khi], vox);
-                                }
-                                acc[m] = fmaf(ampu, vox, acc[m]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-                __syncwarp();
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < MZ; m++) {
-            const int dz = lane + 32 * m;
-            if (dz < izn)
-                store_from_float(image, (size_t)(iz0 + dz) * nxy + (size_t)iy * g.nx + ix, on ? acc[m] * scale : 0.0f,
-                                 out_dtype);
-        }
-    }
-}
-
 // ps = proj * ampv (the axial amplitude the reference applies to the backprojected
 // view in place, geom/cbct/cbct_back.c:196-214), into scratch.
-// Four resident blocks per SM (registers capped at 64): measured on B200 at config 2,
-// DD 110 -> 100 ms and SF 143 -> 104 ms against the uncapped 80-118 registers.
-template <int METHOD, int MZ, bool VEC, int SRC = kSrcScaled, bool SUM = false>
-__global__ void __launch_bounds__(256, 4) back_kernel(Geom g, const View *__restrict__ views,
-                                                   const void *__restrict__ ps, const uint8_t *__restrict__ map,
-                                                   void *__restrict__ image, int out_dtype, int view_begin,
-                                                   int view_stride, int view_count, float scale, int qcap,
-                                                   int *__restrict__ err, const float *__restrict__ ampv,
-                                                   int block_base) {
-    extern __shared__ float smem[];
-    back_block<METHOD, MZ, VEC, SRC, SUM>(g, views, ps, map, image, out_dtype, view_begin, view_stride,
-                                                view_count, scale, qcap, err, ampv, smem, block_base + blockIdx.x);
-}
-
 __global__ void prescale_kernel(const void *__restrict__ proj, int in_dtype, const float *__restrict__ ampv,
                                 float *__restrict__ ps, size_t nuv, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -664,67 +373,12 @@ cudaError_t allow_dynamic_smem(const void *kfn, size_t bytes) {
     return e;
 }
 
-// per warp: the u weights of 32 views and the row buffer; 4 spare floats past the last
-// warp's buffer for the branch-free row reads
-size_t back_smem_bytes(int qcap) { return ((size_t)8 * (32 * 17 + 32 * 8 + qcap) + 4) * sizeof(float); }
-
-template <int METHOD, int MZ, bool VEC, int SRC, bool SUM>
-static cudaError_t launch_back_mz(const Geom &g, const View *views, const void *ps, const float *ampv,
-                                  const uint8_t *map, void *image, int out_dtype, int vb, int vs, int vc, float scale,
-                                  int qcap, int *err, int y_begin, int y_end, cudaStream_t st) {
-    const int tiles_x = (g.nx + 7) / 8;
-    const int blocks = (y_end - y_begin) * tiles_x;
-    if (blocks <= 0) return cudaSuccess;
-    const size_t sm = back_smem_bytes(qcap);
-    auto kfn = back_kernel<METHOD, MZ, VEC, SRC, SUM>;
-    cudaError_t e = allow_dynamic_smem((const void *)kfn, sm);
-    if (e != cudaSuccess) return e;
-    kfn<<<blocks, 256, sm, st>>>(g, views, ps, map, image, out_dtype, vb, vs, vc, scale, qcap, err, ampv,
-                                 y_begin * tiles_x);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_prescale(const void *proj, int in_dtype, const float *ampv, float *ps, size_t nuv, size_t n,
                             cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 32);
     prescale_kernel<<<blocks, 256, 0, st>>>(proj, in_dtype, ampv, ps, nuv, n);
     return cudaGetLastError();
-}
-
-cudaError_t launch_back(int method, int mz, const Geom &g, const View *views, const void *ps, const uint8_t *map,
-                        void *image, int out_dtype, int vb, int vs, int vc, float scale, int qcap, int *err,
-                        cudaStream_t st, bool accumulate, int y_begin, int y_end, int src, const float *ampv) {
-    if (accumulate && (out_dtype != kF32 || scale != 1.0f || src != kSrcScaled)) return cudaErrorInvalidValue;
-    if (src != kSrcScaled && src != kSrcBF16 && src != kSrcF16) return cudaErrorInvalidValue;
-    if (src != kSrcScaled && !ampv) return cudaErrorInvalidValue;
-    if (y_end < 0) y_end = g.ny;
-    if (y_begin < 0 || y_end > g.ny || y_begin > y_end) return cudaErrorInvalidValue;
-    const size_t align = src == kSrcScaled ? 16 : 8;  // one float4, or four 16-bit values, per load
-    const bool vec = (g.nv % 4) == 0 && (reinterpret_cast<uintptr_t>(ps) % align) == 0 &&
-                     (reinterpret_cast<uintptr_t>(ampv) % 16) == 0;
-    // accumulate: the image holds the FP32 view sum of earlier views, which the kernel
-    // continues (separate instantiations, so the plain kernel keeps its registers)
-#define CTSIM_BACK_ARGS g, views, ps, ampv, map, image, out_dtype, vb, vs, vc, scale, qcap, err, y_begin, y_end, st
-#define CTSIM_BACK_CASE(M, Z)                                                                            \
-    if (method == M && mz == Z) {                                                                        \
-        if (accumulate)                                                                                  \
-            return vec ? launch_back_mz<M, Z, true, kSrcScaled, true>(CTSIM_BACK_ARGS)                   \
-                       : launch_back_mz<M, Z, false, kSrcScaled, true>(CTSIM_BACK_ARGS);                 \
-        if (src == kSrcBF16)                                                                             \
-            return vec ? launch_back_mz<M, Z, true, kSrcBF16, false>(CTSIM_BACK_ARGS)                    \
-                       : launch_back_mz<M, Z, false, kSrcBF16, false>(CTSIM_BACK_ARGS);                  \
-        if (src == kSrcF16)                                                                              \
-            return vec ? launch_back_mz<M, Z, true, kSrcF16, false>(CTSIM_BACK_ARGS)                     \
-                       : launch_back_mz<M, Z, false, kSrcF16, false>(CTSIM_BACK_ARGS);                   \
-        return vec ? launch_back_mz<M, Z, true, kSrcScaled, false>(CTSIM_BACK_ARGS)                      \
-                   : launch_back_mz<M, Z, false, kSrcScaled, false>(CTSIM_BACK_ARGS);                    \
-    }
-    CTSIM_BACK_CASE(kDD, 1) CTSIM_BACK_CASE(kDD, 2) CTSIM_BACK_CASE(kDD, 4) CTSIM_BACK_CASE(kDD, 8)
-    CTSIM_BACK_CASE(kTF, 1) CTSIM_BACK_CASE(kTF, 2) CTSIM_BACK_CASE(kTF, 4) CTSIM_BACK_CASE(kTF, 8)
-#undef CTSIM_BACK_CASE
-#undef CTSIM_BACK_ARGS
-    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_prefix(const void *image, int in_dtype, float *xs, int nxy, int nz, bool pairs, int xstride,
@@ -790,32 +444,6 @@ cudaError_t launch_proj(int method, int groups, int rows, bool pairs, const Geom
     return cudaErrorInvalidValue;
 }
 
-// A^T reading the unscaled sinogram (axial amplitude applied on the fly); used by the
-// entry point that allocates nothing (noalloc.cu).
-template <int METHOD, int MZ>
-static cudaError_t launch_back_unscaled_mz(const Geom &g, const View *views, const float *proj, const float *ampv,
-                                           const uint8_t *map, float *image, int vc, int qcap, int *err,
-                                           cudaStream_t st) {
-    const int blocks = g.ny * ((g.nx + 7) / 8);
-    const size_t sm = back_smem_bytes(qcap);
-    auto kfn = back_kernel<METHOD, MZ, false, kSrcF32>;
-    cudaError_t e = allow_dynamic_smem((const void *)kfn, sm);
-    if (e != cudaSuccess) return e;
-    kfn<<<blocks, 256, sm, st>>>(g, views, proj, map, image, kF32, 0, 1, vc, 1.0f, qcap, err, ampv, 0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_back_unscaled(int mz, const Geom &g, const View *views, const float *proj, const float *ampv,
-                                 const uint8_t *map, float *image, int vc, int qcap, int *err, cudaStream_t st) {
-    switch (mz) {
-    case 1: return launch_back_unscaled_mz<kDD, 1>(g, views, proj, ampv, map, image, vc, qcap, err, st);
-    case 2: return launch_back_unscaled_mz<kDD, 2>(g, views, proj, ampv, map, image, vc, qcap, err, st);
-    case 4: return launch_back_unscaled_mz<kDD, 4>(g, views, proj, ampv, map, image, vc, qcap, err, st);
-    case 8: return launch_back_unscaled_mz<kDD, 8>(g, views, proj, ampv, map, image, vc, qcap, err, st);
-    }
-    return cudaErrorInvalidValue;
-}
-
 // ---------------------------------------------------------------------------
 // Batched launches.  One persistent grid (the resident blocks of the whole GPU) walks
 // the flat block list of up to kBatchMax tasks -- plans of different geometries -- and
@@ -841,25 +469,6 @@ __global__ void __launch_bounds__(kProjMaxThreads) proj_batch_kernel(const __gri
     }
 }
 
-template <int METHOD, int MZ, bool VEC, bool LOWP, int SRC>
-__global__ void __launch_bounds__(256) back_batch_kernel(const __grid_constant__ BackBatch b) {
-    extern __shared__ float smem_batch[];
-    for (int blk = blockIdx.x; blk < b.total; blk += gridDim.x) {
-        int lo = 0, hi = b.n - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (b.t[mid].first <= blk) lo = mid; else hi = mid - 1;
-        }
-        const BackTask &T = b.t[lo];
-        back_block<METHOD, MZ, VEC, SRC>(T.g, T.views, T.ps, T.map, T.image, LOWP ? T.out_dtype : kF32, T.vb, T.vs,
-                                         T.vc, T.scale, T.qcap, T.err, T.ampv, smem_batch, blk - T.first);
-        // the per-warp row buffers are laid out with the task's own stride, so a warp may
-        // not start the next item (possibly another task) while its neighbours still work
-        __syncthreads();
-    }
-}
-
-int back_task_blocks(const Geom &g) { return g.ny * ((g.nx + 7) / 8); }
 int proj_row_threads_of(int nv) { return proj_row_threads(nv); }
 
 int persistent_grid(const void *kernel, int threads, size_t smem, int total) {
@@ -886,33 +495,6 @@ cudaError_t launch_proj_batch(int method, int groups, int row_threads, bool pair
     CTSIM_PB_CASE(kDD, 1) CTSIM_PB_CASE(kDD, 2) CTSIM_PB_CASE(kDD, 4) CTSIM_PB_CASE(kDD, 8)
     CTSIM_PB_CASE(kTF, 1) CTSIM_PB_CASE(kTF, 2) CTSIM_PB_CASE(kTF, 4) CTSIM_PB_CASE(kTF, 8)
 #undef CTSIM_PB_CASE
-    return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_back_batch(int method, int mz, bool vec, bool lowp, size_t smem, const BackBatch &b,
-                              cudaStream_t st, int src) {
-    if (b.n < 1 || b.total < 1) return cudaSuccess;
-    if (src != kSrcScaled && src != kSrcBF16 && src != kSrcF16) return cudaErrorInvalidValue;
-#define CTSIM_BB_LAUNCH(M, Z, V, S)                                                                   \
-    {                                                                                                 \
-        auto k = lowp ? back_batch_kernel<M, Z, V, true, S> : back_batch_kernel<M, Z, V, false, S>;   \
-        cudaError_t e = allow_dynamic_smem((const void *)k, smem);                                    \
-        if (e != cudaSuccess) return e;                                                               \
-        k<<<persistent_grid((const void *)k, 256, smem, b.total), 256, smem, st>>>(b);                              \
-        return cudaGetLastError();                                                                    \
-    }
-#define CTSIM_BB_CASE(M, Z, V)                                                                        \
-    if (method == M && mz == Z && vec == V) {                                                         \
-        if (src == kSrcBF16) CTSIM_BB_LAUNCH(M, Z, V, kSrcBF16)                                       \
-        if (src == kSrcF16) CTSIM_BB_LAUNCH(M, Z, V, kSrcF16)                                         \
-        CTSIM_BB_LAUNCH(M, Z, V, kSrcScaled)                                                          \
-    }
-    CTSIM_BB_CASE(kDD, 1, true) CTSIM_BB_CASE(kDD, 2, true) CTSIM_BB_CASE(kDD, 4, true) CTSIM_BB_CASE(kDD, 8, true)
-    CTSIM_BB_CASE(kDD, 1, false) CTSIM_BB_CASE(kDD, 2, false) CTSIM_BB_CASE(kDD, 4, false) CTSIM_BB_CASE(kDD, 8, false)
-    CTSIM_BB_CASE(kTF, 1, true) CTSIM_BB_CASE(kTF, 2, true) CTSIM_BB_CASE(kTF, 4, true) CTSIM_BB_CASE(kTF, 8, true)
-    CTSIM_BB_CASE(kTF, 1, false) CTSIM_BB_CASE(kTF, 2, false) CTSIM_BB_CASE(kTF, 4, false) CTSIM_BB_CASE(kTF, 8, false)
-#undef CTSIM_BB_CASE
-#undef CTSIM_BB_LAUNCH
     return cudaErrorInvalidValue;
 }
 
