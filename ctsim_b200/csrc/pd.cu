@@ -3,6 +3,7 @@
 // (geom/cbct/cbct_back_var.c).
 //
 // Layouts (reference MEX conventions): image[iz][iy][ix], proj[view][iu][iv].
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -42,7 +43,7 @@ __device__ __forceinline__ V pdiv_by(V a, float d, float r) {
 // a view's table loads, unpacking and branches over them and puts their loads in flight
 // together.
 //
-// SUM: the FP32 image holds the view sum of earlier view chunks (scale 1), which the
+// sum: the FP32 image holds the view sum of earlier view chunks (scale 1), which the
 // kernel continues in the same view order.  DT: the sinogram's storage type, read as it
 // is (widening to FP32 is exact, so the result equals that of an FP32 copy bit for bit).
 // The image is written as (sum * scale) * scale2.  one: 1.0f (padd_product).
@@ -52,11 +53,12 @@ struct PdArgs {
     void *image;
     int out_dtype, view_begin, view_stride, view_count;
     float scale, scale2, one;
+    bool sum;
 };
 
 // One pass: NP registers of W voxels per lane from slice iz0 (the last ones may lie past
 // the volume: they sample clamped rows and are not stored).  vtab: the warp's view table.
-template <int MODE, int NP, class V, bool SUM, int DT>
+template <int MODE, int NP, class V, int DT>
 __device__ __forceinline__ void pd_pass(const Geom &g, const PdArgs &A, float4 (*vtab)[2], int ix, int iy, int iz0,
                                         bool on) {
     using P = Packed<V>;
@@ -80,7 +82,7 @@ __device__ __forceinline__ void pd_pass(const Geom &g, const PdArgs &A, float4 (
         // (iz + wz) * dz (cbct_back.c:100); back,var: iz, its wz is the view's
         const V iz = P::make([&](int i) { return (float)(iz0 + lane + 32 * (W * p + i)); });
         zc0[p] = VAR ? iz : pmul(padd(iz, P::all(g.wz_pd)), dz);
-        if (SUM)
+        if (A.sum)
             acc[p] = P::make([&](int i) {
                 const int dzi = 32 * (W * p + i);
                 return lane + dzi < izn ? static_cast<const float *>(A.image)[out0 + (size_t)dzi * nxy] : 0.0f;
@@ -186,18 +188,18 @@ __device__ __forceinline__ void pd_pass(const Geom &g, const PdArgs &A, float4 (
 }
 
 // A full pass of MZ 32-voxel blocks, or the shortest one that covers the remaining slices.
-template <int MODE, int NP, class V, bool SUM, int DT>
+template <int MODE, int NP, class V, int DT>
 __device__ __forceinline__ void pd_pass_of(int np, const Geom &g, const PdArgs &A, float4 (*vtab)[2], int ix, int iy,
                                            int iz0, bool on) {
     if constexpr (NP > 1)
         if (np < NP) {
-            pd_pass_of<MODE, NP - 1, V, SUM, DT>(np, g, A, vtab, ix, iy, iz0, on);
+            pd_pass_of<MODE, NP - 1, V, DT>(np, g, A, vtab, ix, iy, iz0, on);
             return;
         }
-    pd_pass<MODE, NP, V, SUM, DT>(g, A, vtab, ix, iy, iz0, on);
+    pd_pass<MODE, NP, V, DT>(g, A, vtab, ix, iy, iz0, on);
 }
 
-template <int MODE, int MZ, class V, bool SUM, int DT>
+template <int MODE, int MZ, class V, int DT>
 __global__ void __launch_bounds__(256, MZ == 1 ? 5 : 4) pd_kernel(Geom g, PdArgs A, const uint8_t *__restrict__ map) {
     constexpr int W = Packed<V>::kWidth, NP = MZ / W;
     const int warp = threadIdx.x >> 5;
@@ -209,9 +211,12 @@ __global__ void __launch_bounds__(256, MZ == 1 ? 5 : 4) pd_kernel(Geom g, PdArgs
     const bool on = map[iy * g.nx + ix] != 0;
     for (int iz0 = 0; iz0 < g.nz; iz0 += 32 * MZ) {
         const int np = min(NP, (g.nz - iz0 + 32 * W - 1) / (32 * W));
-        pd_pass_of<MODE, NP, V, SUM, DT>(np, g, A, vtab[warp], ix, iy, iz0, on);
+        pd_pass_of<MODE, NP, V, DT>(np, g, A, vtab[warp], ix, iy, iz0, on);
     }
 }
+
+// Sinogram bytes of a view chunk.
+constexpr size_t kPdChunkBytes = (size_t)160 << 20;
 
 template <int MODE, int MZ>
 static cudaError_t launch_pd_mz(const Geom &g, const View *views, const void *proj, int in_dtype, const uint8_t *map,
@@ -219,12 +224,25 @@ static cudaError_t launch_pd_mz(const Geom &g, const View *views, const void *pr
                                 bool accumulate, cudaStream_t st) {
     using V = std::conditional_t<MZ == 1, float, f32x2>;
     const int blocks = g.ny * ((g.nx + 7) / 8);
-    auto k = accumulate          ? pd_kernel<MODE, MZ, V, true, kF32>
-             : in_dtype == kBF16 ? pd_kernel<MODE, MZ, V, false, kBF16>
-             : in_dtype == kF16  ? pd_kernel<MODE, MZ, V, false, kF16>
-                                 : pd_kernel<MODE, MZ, V, false, kF32>;
-    const PdArgs A{views, proj, image, out_dtype, vb, vs, vc, scale, scale2, 1.0f};
-    k<<<blocks, 256, 0, st>>>(g, A, map);
+    auto k = in_dtype == kBF16  ? pd_kernel<MODE, MZ, V, kBF16>
+             : in_dtype == kF16 ? pd_kernel<MODE, MZ, V, kF16>
+                                : pd_kernel<MODE, MZ, V, kF32>;
+    // Blocks of a long launch drift apart over the views until the detector columns they read
+    // no longer meet in L2 (a 512^2 x 256 volume: 7.1 ms for 90 views, 70.4 ms for 720).  So an
+    // FP32 image takes a sinogram of more than two chunks chunk by chunk, continuing its sums:
+    // for 720 views of 1.6 MB, 70.4 ms in one launch, 67.1, 60.7, 58.7, 58.2 and 62.3 ms in
+    // chunks of 32, 64, 96, 128 and 192 views (a chunk costs the volume's read and write).
+    const size_t view_bytes = (size_t)g.nu * g.nv * (in_dtype == kF32 ? 4 : 2);
+    const int chunk = std::max(32, (int)(kPdChunkBytes / view_bytes / 32 * 32));
+    const bool split = out_dtype == kF32 && vc > 2 * chunk;
+    for (int c = 0; c < vc;) {
+        const int n = split ? std::min(chunk, vc - c) : vc;
+        const bool last = c + n == vc;
+        const PdArgs A{views, static_cast<const char *>(proj) + (size_t)c * view_bytes, image, out_dtype, vb + c * vs,
+                       vs, n, last ? scale : 1.0f, last ? scale2 : 1.0f, 1.0f, accumulate || c > 0};
+        k<<<blocks, 256, 0, st>>>(g, A, map);
+        c += n;
+    }
     return cudaGetLastError();
 }
 
