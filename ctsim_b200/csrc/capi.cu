@@ -377,14 +377,26 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     CTSIM_ALLOC(p->d_map, mp.size());
     CTSIM_ALLOC(p->d_err, sizeof(int));
     p->xs_holds_pairs = forward_pairs(nxy, G.nz);
-    // the staged projector: as many columns per stage as leave room for two blocks on an SM
+    // The staged projector: as many columns per stage as leave room for two blocks on an SM, or,
+    // where the detector is short (two row pairs, 64 registers a thread), for three: 512^2 x 256,
+    // 60 views of 128 rows, 24 columns 7.88 ms, 16 columns 6.85 ms.
     p->fwd_sgroups = 1;
     auto staged_bytes = [&](int slots) {
         return proj_staged_smem_bytes(G.nv, std::max(G.nx, G.ny), g.xstride, p->fwd_sgroups, slots);
     };
     p->fwd_slots = 32;
-    while (p->fwd_slots > 8 && staged_bytes(p->fwd_slots) > 110 * 1024) p->fwd_slots -= 8;
-    p->fwd_staged = (g.taps <= 3 || !p->xs_holds_pairs) && proj_slots_valid(g.xstride, p->fwd_slots) &&
+    const size_t room = (size_t)(G.nv <= 128 ? 72 : 110) * 1024;
+    while (p->fwd_slots > 8 && staged_bytes(p->fwd_slots) > room) p->fwd_slots -= 8;
+    // It is the default where a row reaches at most three voxels (faster at every size
+    // measured, 2.08 -> 0.90 ms at 128^2 x 64, 5.6 -> 4.9 ms at 100^2 x 1500) and, since a row takes
+    // its voxels one by one, for longer rows on columns short enough to leave many on an SM.
+    // DD A, staged against paired sums: 128^2 x 64, rows of 4, 5 and 7 voxels 1.14, 1.34, 1.60
+    // against 2.27 ms; 100^2 x 256 0.45, 0.52, 0.44 against 0.68; 100^2 x 600 2.6, 2.1, 2.0
+    // against 2.1, 1.6, 1.7.  Against single sums: 300^2 x 600 5.4, 4.7, 4.5 against 6.4, 5.5, 5.7
+    // ms; 300^2 x 800 7.9, 7.3, 6.0 against 7.0, 7.9, 6.0; 200^2 x 1200 8.2, 7.4, 6.8 against 4.7,
+    // 3.9, 3.9.
+    const bool long_rows = g.taps <= 8 && G.nz <= (p->xs_holds_pairs ? 256 : 600);
+    p->fwd_staged = (g.taps <= 3 || long_rows) && proj_slots_valid(g.xstride, p->fwd_slots) &&
                     staged_bytes(p->fwd_slots) <= 200 * 1024;
     p->fwd_pairs = p->xs_holds_pairs && !p->fwd_staged;
     if (p->fwd_ok)

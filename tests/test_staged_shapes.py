@@ -84,3 +84,21 @@ def test_wide_footprints_and_map():
     for m in ("dd", "tf"):
         got = plan.project(torch.from_numpy(x).cuda(), m).cpu().numpy()
         assert _rel(got, oracle_cbct(f"proj,{m}", g, x)) <= REL_L2, m
+
+
+@pytest.mark.parametrize("nz,nv,dz,dv,layout", [(60, 41, 1.0, 1.6, 3), (96, 40, 0.5, 1.9, 3), (256, 70, 0.5, 3.0, 3),
+                                               (257, 70, 0.5, 3.0, 2), (120, 20, 0.2, 3.2, 2), (301, 128, 1.0, 3.0, 2)])
+def test_default_route_at_its_lines(nz, nv, dz, dv, layout):
+    """The default projector on both sides of the lines between staged columns and paired sums
+    (voxels per row, slices) is within the parity tolerance of the oracle."""
+    import torch
+    from ctsim_b200.projector import Plan
+    from oracle.bindings import oracle_cbct
+    g = _geom(nz, nv, dz, dv)
+    plan = Plan(g)
+    assert plan.tuning["proj_layout"] == layout
+    x = np.random.default_rng(nz).random(g.image_shape, dtype=np.float32)
+    for m in ("dd", "tf"):
+        got = plan.project(torch.from_numpy(x).cuda(), m).cpu().numpy()
+        plan.check()
+        assert _rel(got, oracle_cbct(f"proj,{m}", g, x)) <= REL_L2, m
