@@ -31,8 +31,8 @@ __global__ void prescale_kernel(const void *__restrict__ proj, int in_dtype, con
 // * PAIRS: xc[col][k] = (X[k], X[k+1] - X[k]) as float2, with the top pair (X[nz], 0), so
 //   X(s) = X[k] + (s - k) * slope is one aligned 8-byte load and one FMA for 0 <= s <= nz;
 // * single: xc[col][k] = X[k] as float (half the bytes: better when the volume's prefix
-//   does not stay cache-resident; measured on B200 at 512^2 x 256), columns xstride =
-//   prefix_stride(nz) floats apart, with X[nz] repeated above X[nz] up to the stride.
+//   does not stay cache-resident; measured on B200 at 512^2 x 256), columns xstride
+//   (column_stride) floats apart, with X[nz] repeated above X[nz] up to the stride.
 // 32 columns per block; a 32x32 tile is transposed through shared memory so that the
 // image reads and the prefix writes are coalesced.
 // ---------------------------------------------------------------------------
