@@ -63,6 +63,9 @@ __device__ __forceinline__ float lds_ordered(uint32_t a) {
     return v;
 }
 
+// Detector rows up to which voxels may take their rows without a loop.
+constexpr int kLoopFreeRows = 8192;
+
 // The work of one block (8 columns of one row iy), as a device function: the plain
 // kernel runs it for blockIdx.x, the batched kernel for each of its work items.
 // one: 1.0f (padd_product).
@@ -82,8 +85,10 @@ __device__ __forceinline__ void back_block(const Geom &g, const View *__restrict
     float *wtab = smem + warp * (32 * kWS + 32 * 8 + qcap);  // [32 views][17] u weights of the view chunk
     // [32 views] per-view scalars of the chunk, written by the view's own lane: {ampu, zinc, vstart,
     // nb | path << 8 | 128-row steps << 16}, {address of row rbase of the first detector column (low,
-    // high word), qadj, r_hi - rbase | r_hi << 16}; path 0: no rows.  Entry 16 of the view's weights is
-    // the element offset of that row in ampv.  qadj: row k of Q is at shared address qadj + 4 *
+    // high word), qadj, r_hi - rbase | r_hi << 16}; path 0: no rows.  A half word holds every r_hi - rbase
+    // (below qcap, which the block's shared memory holds eight times), and r_hi up to kLoopFreeRows
+    // rows; taller detectors take path 5, which reads r_hi modulo 2^16.  Entry 16 of the view's weights
+    // is the element offset of that row in ampv.  qadj: row k of Q is at shared address qadj + 4 *
     // bits(k + 2^23) (mod 2^32)
     float4 *vtab = reinterpret_cast<float4 *>(wtab + 32 * kWS);  // 16-byte aligned: 32 * 17 * 4 = 2176
     float *Q = wtab + 32 * kWS + 32 * 8;                         // [qcap] q per row
@@ -143,11 +148,12 @@ __device__ __forceinline__ void back_block(const Geom &g, const View *__restrict
                         if (r_lo <= r_hi) {
                             const int rbase = r_lo & ~3;
                             // A voxel's vmax - vmin is zinc within 1.5 float ulps of nv (< 2^-10 for nv <=
-                            // 8192), so below 1 and 2 by a margin every voxel of the view covers at most
-                            // two or three rows: paths 1 and 2, and 3 and 4 where the detector clips some
-                            // voxel of the pass.
+                            // kLoopFreeRows), so below 1 and 2 by a margin every voxel of the view covers
+                            // at most two or three rows: paths 1 and 2, and 3 and 4 where the detector
+                            // clips some voxel of the pass.
                             constexpr float kMargin = 1.0f / 256.0f;
                             int path = zinc < 1.0f - kMargin ? 1 : zinc < 2.0f - kMargin ? 2 : kGeneric;
+                            if (g.nv > kLoopFreeRows) path = kGeneric;
                             if (path != kGeneric && !(a0u > 0.0f && b1u < fnv)) path += 2;
                             if (r_hi - rbase + 1 > qcap) {  // rows rbase..r_hi must fit
                                 atomicOr(err, 1);
@@ -310,7 +316,9 @@ __device__ __forceinline__ void back_block(const Geom &g, const View *__restrict
                                     khi = klo + (kMaxRowsV - 1);
                                     fhi = fadd(flo, (float)(kMaxRowsV - 1));
                                 }
-                                khi = min(khi, r_hi);  // only after a row-buffer overflow (flagged above)
+                                // at most r_hi, from its low half (a pass spans fewer than 2^15 rows): only
+                                // after a row-buffer overflow (flagged above)
+                                khi = min(khi, klo + (int)(short)(r_hi - klo));
                                 float vox = 0.0f;
                                 if (klo == khi) {
                                     vox = fsub(vmax, vmin) * qb(klo);
