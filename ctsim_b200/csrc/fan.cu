@@ -158,18 +158,22 @@ __device__ __forceinline__ double fan_contribution(int iu, int lo, int hi, float
 
 // Bin iu of view v by four consecutive lanes: row by row the pixels whose centre projects to
 // within `reach` bins of the bin -- u(x) >= c is linear in x, x (cos - r sin) >= r (sad + y cos)
-// + y sin with r the tangent at u = c -- four at a time, their contributions added in order by
-// all four lanes alike.
+// + y sin with r the tangent at u = c (an edge 90 degrees off the axis and more bounds nothing)
+// -- four at a time, their contributions added in order by all four lanes alike.
 template <bool TF>
 __device__ __forceinline__ float fan_gather(const FanGeom &g, const FanView &v, const float *__restrict__ image, int iu,
                                             float reach) {
     const int q = threadIdx.x & (kFanLanes - 1);
-    auto tangent = [&](float u) {
-        const float r = (u + g.wu - 0.5f) / g.sdd_du;
-        return g.det == 1 ? r : tanf(r);
+    // tangent r and slope a at u; both 0 where the edge bounds nothing
+    auto edge = [&](float u, float &r, float &a) {
+        r = (u + g.wu - 0.5f) / g.sdd_du;
+        const bool bounds = g.det == 1 || fabsf(r) < 1.57f;
+        if (g.det != 1) r = bounds ? tanf(r) : 0.0f;
+        a = bounds ? v.cos_a - r * v.sin_a : 0.0f;
     };
-    const float r0 = tangent((float)iu - reach), r1 = tangent((float)(iu + 1) + reach);
-    const float a0 = v.cos_a - r0 * v.sin_a, a1 = v.cos_a - r1 * v.sin_a;
+    float r0, a0, r1, a1;
+    edge((float)iu - reach, r0, a0);
+    edge((float)(iu + 1) + reach, r1, a1);
     // pixels [first, last) of a row that may meet a0 x >= b0 and a1 x <= b1 (one pixel of slack)
     auto range = [&](int iy, int &first, int &last) {
         const float yc = ((float)iy + g.wy) * g.dy;
