@@ -65,6 +65,7 @@ struct ctsim_plan {
     float *d_ampv = nullptr;
     uint8_t *d_map = nullptr;
     float *d_xs = nullptr;   // voxel columns or their prefix sums [nx*ny][g.xstride] (or pairs [nx*ny][nz+1][2]) -- forward scratch
+    uint8_t *d_xstate = nullptr;  // per voxel column: its map entry and whether its voxels are finite (staged projector)
     float *d_ps = nullptr;   // sinogram scaled by ampv [noviews][nu][nv] -- backprojector scratch
     int *d_err = nullptr;
     size_t bytes = 0;
@@ -152,6 +153,7 @@ static void free_plan(ctsim_plan *p) {
     ctsim_plan_release(p, p->d_ampv);
     ctsim_plan_release(p, p->d_map);
     ctsim_plan_release(p, p->d_xs);
+    ctsim_plan_release(p, p->d_xstate);
     ctsim_plan_release(p, p->d_ps);
     ctsim_plan_release(p, p->d_err);
     delete p;
@@ -399,9 +401,11 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     p->fwd_staged = (g.taps <= 3 || long_rows) && proj_slots_valid(g.xstride, p->fwd_slots) &&
                     staged_bytes(p->fwd_slots) <= 200 * 1024;
     p->fwd_pairs = p->xs_holds_pairs && !p->fwd_staged;
-    if (p->fwd_ok)
+    if (p->fwd_ok) {
         CTSIM_ALLOC(p->d_xs, sizeof(float) * (size_t)nxy *
                                  std::max(g.xstride, p->xs_holds_pairs ? 2 * (G.nz + 1) : 0));
+        CTSIM_ALLOC(p->d_xstate, (size_t)nxy);
+    }
     // the backprojection scratch (an FP32 copy of the sinogram times ampv) is allocated on
     // first use (ensure_scratch): BF16/FP16 sinograms and CTSIM_INPUT_SCALED residuals are
     // read as they are and never need it
@@ -477,7 +481,9 @@ static ctsim_status ensure_scratch(ctsim_plan *p, cudaStream_t st) {
 // column prefix sums.
 static cudaError_t prepare_image(const ctsim_plan *p, const void *d_image, int image_dtype, cudaStream_t st) {
     const int nxy = p->g.nx * p->g.ny;
-    if (p->fwd_staged) return launch_columns(d_image, image_dtype, p->d_xs, nxy, p->g.nz, p->g.xpad, p->g.xstride, st);
+    if (p->fwd_staged)
+        return launch_columns(d_image, image_dtype, p->d_map, p->d_xs, p->d_xstate, nxy, p->g.nz, p->g.xpad,
+                              p->g.xstride, st);
     return launch_prefix(d_image, image_dtype, p->d_xs, nxy, p->g.nz, p->fwd_pairs, p->g.xstride, st);
 }
 
@@ -498,8 +504,8 @@ static ctsim_status plan_project(ctsim_plan *p, int method, const void *d_image,
     if (prefix && (e = prepare_image(p, d_image, image_dtype, st)) != cudaSuccess) return cuda_fail(e, "prefix kernel");
     if (p->fwd_staged)
         e = launch_proj_staged(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_sgroups, p->fwd_slots, p->g, p->d_views,
-                               p->d_xs, p->d_ampv, p->d_map, d_proj, proj_dtype, view_begin, view_stride, view_count,
-                               p->margin, p->d_err, st);
+                               p->d_xs, p->d_ampv, p->d_xstate, d_proj, proj_dtype, view_begin, view_stride,
+                               view_count, p->margin, p->d_err, st);
     else
         e = launch_proj(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_groups, p->fwd_rows, p->fwd_pairs, p->g,
                         p->d_views, p->d_xs, p->d_ampv, p->d_map, d_proj, proj_dtype, view_begin, view_stride,
@@ -1413,6 +1419,7 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
                 T.xs = p->d_xs;
                 T.ampv = p->d_ampv;
                 T.map = p->d_map;
+                T.state = p->d_xstate;
                 T.proj = it.out;
                 T.out_dtype = it.out_dtype;
                 T.vb = it.view_begin;

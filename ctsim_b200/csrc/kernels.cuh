@@ -62,12 +62,13 @@ bool proj_shape_valid(int nv, int groups, int rows);
 size_t proj_smem_bytes(int nv, int nx, int ny, int groups, int rows);
 // The forward projector with the candidates' voxel columns staged in shared memory
 // (proj_staged.cu): xs holds the image as columns (launch_columns; 16-byte aligned),
-// up to `slots` of them per stage; candidate groups 1, 2, 4 or 8.  A stage wait
-// that runs out sets bit 4 of *err.
-cudaError_t launch_columns(const void *image, int in_dtype, float *xs, int nxy, int nz, int xpad, int xstride,
-                           cudaStream_t st);
+// up to `slots` of them per stage; candidate groups 1, 2, 4 or 8.  state: one byte per column,
+// its place in the map and whether its voxels are finite.  A stage wait that runs out sets bit 4
+// of *err.
+cudaError_t launch_columns(const void *image, int in_dtype, const uint8_t *map, float *xs, uint8_t *state, int nxy,
+                           int nz, int xpad, int xstride, cudaStream_t st);
 cudaError_t launch_proj_staged(int method, int groups, int slots, const Geom &g, const View *views, const float *xs,
-                               const float *ampv, const uint8_t *map, void *proj, int out_dtype, int view_begin,
+                               const float *ampv, const uint8_t *state, void *proj, int out_dtype, int view_begin,
                                int view_stride, int view_count, float margin, int *err, cudaStream_t st);
 size_t proj_staged_smem_bytes(int nv, int nlines, int xstride, int groups, int slots);
 bool proj_slots_valid(int xstride, int slots);
@@ -99,7 +100,7 @@ struct ProjTask {
     const View *views;
     const float *xs;
     const float *ampv;
-    const uint8_t *map;
+    const uint8_t *map, *state;  // state: the staged projector's columns
     void *proj;
     int out_dtype;
     int vb, vs, vc, gx, first;  // view selection, blocks along u, first flat block of the task

@@ -49,17 +49,27 @@ constexpr int kPart = 4;  // detector columns of a consumer warp
 // ---------------------------------------------------------------------------
 // The column layout: col[ix + iy nx][k], k = 0 .. g.xstride - 1, holds g.xpad zeros, the nz
 // voxels, zeros.  A 32 x 32 tile is transposed through shared memory so that the image
-// reads and the column writes are coalesced.
+// reads and the column writes are coalesced.  state[col]: kColumnOn where the map has the
+// column, kColumnNonFinite where a voxel of it is infinite or NaN.
 // ---------------------------------------------------------------------------
+constexpr int kColumnOn = 1, kColumnNonFinite = 2;
+
 __global__ void __launch_bounds__(256) columns_kernel(const void *__restrict__ image, int in_dtype,
-                                                      float *__restrict__ xs, int nxy, int nz, int xpad, int xstride) {
+                                                      const uint8_t *__restrict__ map, float *__restrict__ xs,
+                                                      uint8_t *__restrict__ state, int nxy, int nz, int xpad,
+                                                      int xstride) {
     __shared__ float tile[32][33];
+    __shared__ int non_finite[32];
     const int c0 = blockIdx.x * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    bool bad = false;
+    if (threadIdx.x < 32) non_finite[threadIdx.x] = 0;
     for (int k0 = 0; k0 < xstride; k0 += 32) {
         for (int kk = ty; kk < 32; kk += 8) {
             const int z = k0 + kk - xpad, c = c0 + tx;
-            tile[kk][tx] = (z >= 0 && z < nz && c < nxy) ? load_as_float(image, (size_t)z * nxy + c, in_dtype) : 0.0f;
+            const float x = (z >= 0 && z < nz && c < nxy) ? load_as_float(image, (size_t)z * nxy + c, in_dtype) : 0.0f;
+            tile[kk][tx] = x;
+            bad |= !isfinite(x);
         }
         __syncthreads();
         for (int cc = ty; cc < 32; cc += 8) {
@@ -68,11 +78,15 @@ __global__ void __launch_bounds__(256) columns_kernel(const void *__restrict__ i
         }
         __syncthreads();
     }
+    if (bad) non_finite[tx] = 1;
+    __syncthreads();
+    if (threadIdx.x < 32 && c0 + tx < nxy)
+        state[c0 + tx] = (map[c0 + tx] ? kColumnOn : 0) | (non_finite[tx] ? kColumnNonFinite : 0);
 }
 
-cudaError_t launch_columns(const void *image, int in_dtype, float *xs, int nxy, int nz, int xpad, int xstride,
-                           cudaStream_t st) {
-    columns_kernel<<<(nxy + 31) / 32, 256, 0, st>>>(image, in_dtype, xs, nxy, nz, xpad, xstride);
+cudaError_t launch_columns(const void *image, int in_dtype, const uint8_t *map, float *xs, uint8_t *state, int nxy,
+                           int nz, int xpad, int xstride, cudaStream_t st) {
+    columns_kernel<<<(nxy + 31) / 32, 256, 0, st>>>(image, in_dtype, map, xs, state, nxy, nz, xpad, xstride);
     return cudaGetLastError();
 }
 
@@ -163,11 +177,12 @@ constexpr int kRing = 3, kProducers = 3;
 // before stage i + kProducers tells that stage's slot one phase back from two only if the
 // use before the last one, i + kProducers - 2 kRing, is among those.
 static_assert(kProducers <= kRing, "a ring shorter than the producers aliases the phases of a slot");
+constexpr int kStageLast = 1, kStageNonFinite = 2;
 struct StagedRing {
     uint64_t full[kRing], empty[kRing];
     int count[kRing][16];  // entries of (column part, candidate group)
     int pairs[kRing];      // row pairs that the stage's entries reach, counted from the block's first
-    int last[kRing];       // the item's last stage
+    int flags[kRing];      // kStageLast: the item's last stage; kStageNonFinite: some column is not finite
     // a producer's or a consumer's wait ran out: read by its own role between two of the role's
     // barriers, where nobody sets it, so that all warps of the role stop at the same item
     int fail_producer, fail_consumer;
@@ -282,8 +297,10 @@ __device__ __forceinline__ int candidate_lines(const Geom &g, const View &v, int
 // volume the taps read the zeros of the layout.  xadj: the column's shared-memory address
 // minus 4 * 0x4B000000 (mod 2^32), so that the word of voxel floor(s) is at xadj + 4 * bits(s
 // + xpad + 2^23 rounded down).  The overlaps are formed from k + 1 - s (one rounding) and
-// the extent's length dl = 1 / zinc, so they stay accurate far up the column.
-template <int TAPS>
+// the extent's length dl = 1 / zinc, so they stay accurate far up the column.  SAFE: a voxel
+// that the extent does not reach counts as 0 whatever its value (an infinity times overlap 0
+// would be NaN).
+template <int TAPS, bool SAFE>
 __device__ __forceinline__ f32x2 staged_rows(uint32_t xadj, f32x2 f, float pa, float pb, float dl, float n, int taps) {
     using P = Packed<f32x2>;
     const f32x2 s01 = P::make([&](int i) { return __saturatef(__fmaf_rn(P::get(f, i), pa, pb)); });
@@ -293,27 +310,32 @@ __device__ __forceinline__ f32x2 staged_rows(uint32_t xadj, f32x2 f, float pa, f
     uint32_t ad[2];
 #pragma unroll
     for (int i = 0; i < 2; i++) ad[i] = xadj + (__float_as_uint(P::get(t, i)) << 2);
-    auto tap = [&](int k) { return P::make([&](int i) { return lds_f32(ad[i] + 4u * k); }); };
+    auto tap = [&](int k, f32x2 overlap) {
+        return P::make([&](int i) {
+            const float x = lds_f32(ad[i] + 4u * k);
+            return !SAFE || P::get(overlap, i) > 0.0f ? x : 0.0f;
+        });
+    };
     f32x2 rem = psub(P::all(dl), a);
-    if (TAPS == 2) return pfma(rem, tap(1), pmul(a, tap(0)));
-    const f32x2 one = P::all(1.0f);
+    if (TAPS == 2) return pfma(rem, tap(1, rem), pmul(a, tap(0, a)));
     if (TAPS == 3) {
         const f32x2 b = P::make([&](int i) { return fminf(P::get(rem, i), 1.0f); });
-        return pfma(psub(rem, b), tap(2), pfma(b, tap(1), pmul(a, tap(0))));
+        rem = psub(rem, b);
+        return pfma(rem, tap(2, rem), pfma(b, tap(1, b), pmul(a, tap(0, a))));
     }
-    f32x2 r = pmul(a, tap(0));
+    f32x2 r = pmul(a, tap(0, a));
     for (int k = 1; k < taps; k++) {  // extents of two voxels and more
         const f32x2 b = P::make([&](int i) { return fminf(P::get(rem, i), 1.0f); });
-        r = pfma(b, tap(k), r);
+        r = pfma(b, tap(k, b), r);
         rem = psub(rem, b);
     }
     return r;
 }
 
 // The entries at shared addresses e, e + step, ... < end over the first NA of the warp's
-// row pairs, added with the weights of the warp's kPart detector columns (0 where the
-// footprint does not reach).
-template <int NP, int NA, int TAPS>
+// row pairs, added with the weights of the warp's kPart detector columns (-0 where the
+// footprint does not reach: SAFE adds nothing there).
+template <int NP, int NA, int TAPS, bool SAFE = false>
 __device__ __forceinline__ void staged_entries(f32x2 (&acc)[kPart][NP], const f32x2 (&frow)[NP], uint32_t e,
                                                uint32_t end, uint32_t step, float n, int taps) {
     float4 next = lds_f32x4(e);
@@ -323,9 +345,19 @@ __device__ __forceinline__ void staged_entries(f32x2 (&acc)[kPart][NP], const f3
         f32x2 r[NA], w[kPart];
         lds_2x2(e + 16u, w[0], w[1]);
         lds_2x2(e + 32u, w[2], w[3]);
+        if constexpr (SAFE) {  // pair by pair: rare, and no more registers than the others
+#pragma unroll
+            for (int p = 0; p < NA; p++) {
+                const f32x2 v = staged_rows<TAPS, true>(__float_as_uint(prm.w), frow[p], prm.x, prm.y, prm.z, n, taps);
+#pragma unroll
+                for (int j = 0; j < kPart; j++)
+                    if (__float_as_uint(w[j].x) != 0x80000000u) acc[j][p] = pfma(w[j], v, acc[j][p]);
+            }
+            continue;
+        }
 #pragma unroll
         for (int p = 0; p < NA; p++)
-            r[p] = staged_rows<TAPS>(__float_as_uint(prm.w), frow[p], prm.x, prm.y, prm.z, n, taps);
+            r[p] = staged_rows<TAPS, false>(__float_as_uint(prm.w), frow[p], prm.x, prm.y, prm.z, n, taps);
 #pragma unroll
         for (int p = 0; p < NA; p++)
 #pragma unroll
@@ -335,7 +367,7 @@ __device__ __forceinline__ void staged_entries(f32x2 (&acc)[kPart][NP], const f3
 
 // u weights of detector columns c0 .. c0 + kPart - 1 (footprint scaled by scl): u_weight of
 // common.cuh, with a trapezoid's two divisions replaced by r0 and r1 (half the reciprocals
-// of its ramps) and its squares' differences formed as (a - b)(a + b).
+// of its ramps) and its squares' differences formed as (a - b)(a + b); -0 off the footprint.
 template <int METHOD>
 __device__ __forceinline__ void staged_weights(const ColumnFP &fp, float scl, float r0, float r1, int c0,
                                                float (&w)[kPart]) {
@@ -353,7 +385,7 @@ __device__ __forceinline__ void staged_weights(const ColumnFP &fp, float scl, fl
             xr = fminf(br, fp.p3);
             v += xr > xl ? ((xr - xl) * ((fp.p3 - xl) + (fp.p3 - xr))) * r1 : 0.0f;
         }
-        w[j] = c0 + j >= fp.iumin && c0 + j <= fp.iumax ? v * scl : 0.0f;
+        w[j] = c0 + j >= fp.iumin && c0 + j <= fp.iumax ? v * scl : -0.0f;
     }
 }
 
@@ -363,7 +395,7 @@ struct StagedItem {
     const Geom *g;
     const View *views;
     const float *xs, *ampv;
-    const uint8_t *map;
+    const uint8_t *state;  // of the columns (columns_kernel)
     void *proj;
     int *err;
     int out_dtype, view_begin, view_stride, bx, by, bz;
@@ -425,7 +457,7 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
     unsigned out_parity = 0;
     for (int i = warp; i < nstages; i += kProducers, my.advance(kProducers)) {
         const int c = i * per + lane;
-        bool valid = false;
+        bool valid = false, non_finite = false;
         int na = 0, col = 0, h0 = 1, h1 = 0;  // the parts the footprint touches
         float pa = 0.f, pb = 0.f, dl = 0.f, scl = 0.f;
         ColumnFP fp;
@@ -438,7 +470,8 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
             const int p = line_start[a] + (c - line_off[a]);
             const int ix = rows ? p : a, iy = rows ? a : p;
             col = iy * g.nx + ix;
-            const bool on = I.map[col] != 0;
+            const int state = I.state[col];
+            const bool on = (state & kColumnOn) != 0;
             fp = column_footprint<METHOD, false>(g, v, ix, iy);
             if (on && fp.hit && fp.iumax >= iu0 && fp.iumin <= iu0 + width - 1) {
                 const float b0 = fp.vstart + 0.5f;
@@ -449,6 +482,7 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
                 na = min(max(rhi - mid, mid - 1 - rlo) / 32 + 1 - V.Q0, PB);
                 if (rlo <= rhi && na > 0) {
                     valid = true;
+                    non_finite = (state & kColumnNonFinite) != 0;
                     h0 = (max(fp.iumin, iu0) - iu0) / kPart;
                     h1 = (min(fp.iumax, iu0 + width - 1) - iu0) / kPart;
                     scl = fp.ampu * fp.zinc;
@@ -466,6 +500,7 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
         const float r1 = METHOD == kTF && valid ? 0.5f / (fp.p3 - fp.p2) : 0.0f;
         const unsigned all = __ballot_sync(kFull, valid);
         const unsigned reach = __reduce_max_sync(kFull, valid ? (unsigned)na : 0u);
+        const bool any_non_finite = __any_sync(kFull, non_finite);
         // lanes of this lane's candidate group: (c mod groups) repeats every `groups` lanes
         unsigned same = 1u << (lane & (groups - 1));
         for (int k = groups; k < 32; k <<= 1) same |= same << k;
@@ -501,7 +536,7 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
             }
         if (lane == 0) {
             ring->pairs[my.stage] = (int)reach;
-            ring->last[my.stage] = i == nstages - 1;
+            ring->flags[my.stage] = (i == nstages - 1 ? kStageLast : 0) | (any_non_finite ? kStageNonFinite : 0);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive_expect(&ring->full[my.stage], (unsigned)__popc(all) * (unsigned)xst * 4u);
@@ -556,10 +591,13 @@ __device__ __forceinline__ bool staged_consume(const StagedItem &I, const Staged
         }
         const int count = ring->count[at.stage][part * 4 + grp];
         const int na = wg == 1 ? ring->pairs[at.stage] : (ring->pairs[at.stage] - gwarp + 1) >> 1;  // wg: 1 or 2
-        last = ring->last[at.stage] != 0;
+        const int flags = ring->flags[at.stage];
+        last = (flags & kStageLast) != 0;
         if (count > 0 && na > 0) {
             const uint32_t e = ent + (uint32_t)at.stage * ent_stage, end = e + (uint32_t)count * step;
-            switch (na) {
+            switch (flags & kStageNonFinite ? 0 : na) {
+            // pairs that the stage does not reach add zeros
+            case 0: staged_entries<NP, NP, TAPS, true>(acc, frow, e, end, step, n, taps); break;
             case 1: staged_entries<NP, 1, TAPS>(acc, frow, e, end, step, n, taps); break;
             case 2: staged_entries<NP, NP < 2 ? NP : 2, TAPS>(acc, frow, e, end, step, n, taps); break;
             case 3: staged_entries<NP, NP < 3 ? NP : 3, TAPS>(acc, frow, e, end, step, n, taps); break;
@@ -666,11 +704,11 @@ __device__ __forceinline__ void staged_block(int total, int groups, int parts, i
 template <int METHOD, int NP, int CW, int TAPS>
 __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * StagedRegs<NP, CW>::kLaunch))
     proj_staged_kernel(const __grid_constant__ Geom g, const View *__restrict__ views, const float *__restrict__ xs,
-                       const float *__restrict__ ampv, const uint8_t *__restrict__ map, void *__restrict__ proj,
+                       const float *__restrict__ ampv, const uint8_t *__restrict__ state, void *__restrict__ proj,
                        int out_dtype, int view_begin, int view_stride, float margin, int groups, int parts,
                        int slots, int *__restrict__ err, int ngx, int vc, int total) {
     staged_block<METHOD, NP, CW, TAPS>(total, groups, parts, slots, max(g.nx, g.ny), [&](int blk) {
-        StagedItem I{&g, views, xs, ampv, map, proj, err, out_dtype, view_begin, view_stride, 0, 0, 0, margin};
+        StagedItem I{&g, views, xs, ampv, state, proj, err, out_dtype, view_begin, view_stride, 0, 0, 0, margin};
         const int per = ngx * vc;
         I.bz = blk / per;
         view_grouped_block(blk - I.bz * per, ngx, vc, I.bx, I.by);
@@ -691,7 +729,7 @@ __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * Stag
             if (b.t[m].first <= blk) lo = m; else hi = m - 1;
         }
         const ProjTask &T = b.t[lo];
-        StagedItem I{&T.g, T.views, T.xs, T.ampv, T.map, T.proj, T.err, T.out_dtype, T.vb, T.vs, 0, 0, 0, T.margin};
+        StagedItem I{&T.g, T.views, T.xs, T.ampv, T.state, T.proj, T.err, T.out_dtype, T.vb, T.vs, 0, 0, 0, T.margin};
         const int per = T.gx * T.vc, l = blk - T.first;
         I.bz = l / per;
         view_grouped_block(l - I.bz * per, T.gx, T.vc, I.bx, I.by);
@@ -738,7 +776,7 @@ bool proj_slots_valid(int xstride, int slots) {
     }
 
 cudaError_t launch_proj_staged(int method, int groups, int slots, const Geom &g, const View *views, const float *xs,
-                               const float *ampv, const uint8_t *map, void *proj, int out_dtype, int vb, int vs,
+                               const float *ampv, const uint8_t *state, void *proj, int out_dtype, int vb, int vs,
                                int vc, float margin, int *err, cudaStream_t st) {
     if ((groups != 1 && groups != 2 && groups != 4 && groups != 8) || !proj_slots_valid(g.xstride, slots) ||
         g.xstride % 4 != 0 || g.xpad < 1 || g.taps < 2 || g.xstride < g.nz + g.xpad + g.taps ||
@@ -749,7 +787,7 @@ cudaError_t launch_proj_staged(int method, int groups, int slots, const Geom &g,
     const int ngx = staged_columns(S, g.nu), taps = g.taps, total = ngx * vc * S.split;
     CTSIM_STAGED_SWITCH(proj_staged_kernel,
                         (k<<<persistent_grid((const void *)k, nt, sm, total), nt, sm, st>>>(
-                            g, views, xs, ampv, map, proj, out_dtype, vb, vs, margin, S.groups, S.parts, slots, err, ngx,
+                            g, views, xs, ampv, state, proj, out_dtype, vb, vs, margin, S.groups, S.parts, slots, err, ngx,
                             vc, total)));
     return cudaErrorInvalidValue;
 }

@@ -93,7 +93,7 @@ def hbm_footprint(req: ReconRequest) -> int:
     reach = g.detSpacing[1] / g.reconSpacing[2] * (g.SAD + math.hypot(g.nx * g.reconSpacing[0], g.ny *
                                                                       g.reconSpacing[1])) / g.SDD
     xs = 4 * g.nx * g.ny * max(2 * (g.nz + 4), g.nz + 2 * int(reach + 1) + 8)
-    plan = xs + 4 * g.nu * g.nv + g.nx * g.ny + 64 * g.noViews + 4096
+    plan = xs + 4 * g.nu * g.nv + 2 * g.nx * g.ny + 64 * g.noViews + 4096
     fdk = s * pix + 4 * g.nu * g.nv + 12 * L + 4 * g.nu * g.noViews + 4096  # filtered sinogram + tables
     image = 4 * vox
     if req.kind == "fdk":
