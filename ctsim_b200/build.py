@@ -13,7 +13,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libctsim_b200.so")
-SOURCES = ["kernels.cu", "proj_staged.cu", "back.cu", "pd.cu", "capi.cu", "noalloc.cu", "fdk.cu", "pwls.cu", "sino.cu", "fan.cu"]
+SOURCES = ["kernels.cu", "proj_staged.cu", "proj_sums.cu", "back.cu", "pd.cu", "capi.cu", "noalloc.cu", "fdk.cu", "pwls.cu",
+           "sino.cu", "fan.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 FLAGS = [

@@ -77,8 +77,9 @@ struct ctsim_plan {
     int fwd_sgroups = 1;     // candidate groups of the staged forward projector (tunable)
     int fwd_rows = 32;       // row threads per group of the unstaged forward projector (tunable)
     bool fwd_pairs = false;  // prefix sums stored as (X, slope) pairs (tunable)
-    bool fwd_staged = false; // voxel columns staged in shared memory (tunable)
-    int fwd_slots = 16;      // columns per stage buffer of the staged projector (tunable)
+    bool fwd_staged = false; // columns staged in shared memory (tunable)
+    bool fwd_columns = false;  // the staged form: voxel columns (proj_staged.cu) or prefix columns (proj_sums.cu)
+    int fwd_slots = 8;       // columns per stage of the staged projector (tunable)
     bool xs_holds_pairs = false;  // the prefix scratch was sized for pairs
     bool fwd_ok = true;
     std::string fwd_reason;
@@ -169,6 +170,23 @@ static int back_qcap_for(const ctsim_plan *p, int mz) {
     return (rows + 127) / 128 * 128;
 }
 static bool back_mz_fits(const ctsim_plan *p, int mz) { return back_smem_bytes(back_qcap_for(p, mz)) <= 200 * 1024; }
+
+// Shared memory of layout 3 with `slots` columns per stage, in the plan's form and with its groups.
+static size_t staged_bytes(const ctsim_plan *p, int slots) {
+    const ctsim_geom &G = p->geom;
+    return p->fwd_columns ? proj_staged_smem_bytes(G.nv, std::max(G.nx, G.ny), p->g.xstride, p->fwd_sgroups, slots)
+                          : proj_sums_smem_bytes(G.nv, G.nx, G.ny, p->g.xstride, p->fwd_groups, p->fwd_rows, slots);
+}
+static bool staged_fits(const ctsim_plan *p, int slots) {
+    return proj_slots_valid(p->g.xstride, slots) && staged_bytes(p, slots) <= 200 * 1024;
+}
+// Columns per stage of a launch over voxel columns: what was asked for, as far as it is used (32) and
+// three stages of it fit.
+static int staged_slots(const ctsim_plan *p) {
+    int slots = std::min(p->fwd_slots, 32);
+    while (slots > 1 && !staged_fits(p, slots)) slots--;
+    return slots;
+}
 
 extern "C" ctsim_status ctsim_plan_create(const ctsim_geom *geom, const double *betas, const float *couchz,
                                           const bool *map, ctsim_plan **out) {
@@ -307,12 +325,28 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     {
         // longest extent of a detector row in voxels (the farthest columns): `taps` voxels from
         // the one its lower edge lies in, and the zeros below voxel 0 that an extent clamped
-        // there may cover
+        // there may cover (staged voxel columns)
         const double len = (double)G.dv / G.dz * ((double)G.sad + rmax) / G.sdd * 1.0001 + 1e-6;
         const int whole = (int)std::min(std::floor(len), 1e6);
         g.xpad = whole + 1;
         g.taps = whole + 2;
+        // What layout 3 stages: voxel columns where a row reaches at most three voxels (faster at
+        // every size measured, 2.08 -> 0.90 ms at 128^2 x 64, 5.6 -> 4.9 ms at 100^2 x 1500) and,
+        // since a row takes its voxels one by one, for rows of up to eight on short columns.  DD A,
+        // voxel columns against paired sums on volumes whose pairs stay cache-resident: 128^2 x 64,
+        // rows of 4, 5 and 7 voxels 1.14, 1.34, 1.60 against 2.27 ms; 100^2 x 256 0.45, 0.52, 0.44
+        // against 0.68; 100^2 x 600 2.6, 2.1, 2.0 against 2.1, 1.6, 1.7.  On larger volumes against
+        // prefix columns, rows of 2.1, 3.2 and 4 voxels at the axis: 512^2 x 128, 16 views 1.51, 1.43,
+        // 1.54 against 1.85, 1.84, 1.83 ms; 512^2 x 256 2.23, 2.51, 2.40 against 2.21, 1.96, 1.95; 300^2
+        // x 400 1.52, 1.25, 1.55 against 1.07, 1.05, 1.09.
+        p->xs_holds_pairs = forward_pairs(nxy, G.nz);
+        p->fwd_sgroups = 1;
         g.xstride = column_stride(G.nz, g.xpad, g.taps);
+        p->fwd_columns = g.taps <= 3 || (g.taps <= 8 && G.nz <= (p->xs_holds_pairs ? 256 : 128));
+        if (!p->fwd_columns || !staged_fits(p, 8)) {
+            p->fwd_columns = false;
+            g.xstride = column_stride(G.nz, 1, 1);
+        }
     }
     const double umm = std::max(std::fabs((double)g.wu * G.du), std::fabs(((double)G.nu - 1 + g.wu) * G.du)) + G.du;
     double stretch = G.detector_type == 1 ? 1.0 + (umm / G.sdd) * (umm / G.sdd) : 1.0;
@@ -378,28 +412,16 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     CTSIM_ALLOC(p->d_ampv, sizeof(float) * ampv.size());
     CTSIM_ALLOC(p->d_map, mp.size());
     CTSIM_ALLOC(p->d_err, sizeof(int));
-    p->xs_holds_pairs = forward_pairs(nxy, G.nz);
-    // The staged projector: as many columns per stage as leave room for two blocks on an SM, or,
-    // where the detector is short (two row pairs, 64 registers a thread), for three: 512^2 x 256,
-    // 60 views of 128 rows, 24 columns 7.88 ms, 16 columns 6.85 ms.
-    p->fwd_sgroups = 1;
-    auto staged_bytes = [&](int slots) {
-        return proj_staged_smem_bytes(G.nv, std::max(G.nx, G.ny), g.xstride, p->fwd_sgroups, slots);
-    };
-    p->fwd_slots = 32;
-    const size_t room = (size_t)(G.nv <= 128 ? 72 : 110) * 1024;
-    while (p->fwd_slots > 8 && staged_bytes(p->fwd_slots) > room) p->fwd_slots -= 8;
-    // It is the default where a row reaches at most three voxels (faster at every size
-    // measured, 2.08 -> 0.90 ms at 128^2 x 64, 5.6 -> 4.9 ms at 100^2 x 1500) and, since a row takes
-    // its voxels one by one, for longer rows on columns short enough to leave many on an SM.
-    // DD A, staged against paired sums: 128^2 x 64, rows of 4, 5 and 7 voxels 1.14, 1.34, 1.60
-    // against 2.27 ms; 100^2 x 256 0.45, 0.52, 0.44 against 0.68; 100^2 x 600 2.6, 2.1, 2.0
-    // against 2.1, 1.6, 1.7.  Against single sums: 300^2 x 600 5.4, 4.7, 4.5 against 6.4, 5.5, 5.7
-    // ms; 300^2 x 800 7.9, 7.3, 6.0 against 7.0, 7.9, 6.0; 200^2 x 1200 8.2, 7.4, 6.8 against 4.7,
-    // 3.9, 3.9.
-    const bool long_rows = g.taps <= 8 && G.nz <= (p->xs_holds_pairs ? 256 : 600);
-    p->fwd_staged = (g.taps <= 3 || long_rows) && proj_slots_valid(g.xstride, p->fwd_slots) &&
-                    staged_bytes(p->fwd_slots) <= 200 * 1024;
+    // Columns per stage.  Voxel columns: as many as leave room for two blocks on an SM, or, where the
+    // detector is short (two row pairs, 64 registers a thread), for three: 512^2 x 256, 60 views of
+    // 128 rows, 24 columns 7.88 ms, 16 columns 6.85 ms.
+    if (p->fwd_columns) {
+        p->fwd_slots = 32;
+        const size_t room = (size_t)(G.nv <= 128 ? 72 : 110) * 1024;
+        while (p->fwd_slots > 8 && staged_bytes(p, p->fwd_slots) > room) p->fwd_slots -= 8;
+    }
+    // staged by default, or paired sums where they stay cache-resident and the rows are long
+    p->fwd_staged = p->fwd_columns || (!p->xs_holds_pairs && staged_fits(p, p->fwd_slots));
     p->fwd_pairs = p->xs_holds_pairs && !p->fwd_staged;
     if (p->fwd_ok) {
         CTSIM_ALLOC(p->d_xs, sizeof(float) * (size_t)nxy *
@@ -481,7 +503,7 @@ static ctsim_status ensure_scratch(ctsim_plan *p, cudaStream_t st) {
 // column prefix sums.
 static cudaError_t prepare_image(const ctsim_plan *p, const void *d_image, int image_dtype, cudaStream_t st) {
     const int nxy = p->g.nx * p->g.ny;
-    if (p->fwd_staged)
+    if (p->fwd_staged && p->fwd_columns)
         return launch_columns(d_image, image_dtype, p->d_map, p->d_xs, p->d_xstate, nxy, p->g.nz, p->g.xpad,
                               p->g.xstride, st);
     return launch_prefix(d_image, image_dtype, p->d_xs, nxy, p->g.nz, p->fwd_pairs, p->g.xstride, st);
@@ -502,12 +524,16 @@ static ctsim_status plan_project(ctsim_plan *p, int method, const void *d_image,
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
     if (prefix && (e = prepare_image(p, d_image, image_dtype, st)) != cudaSuccess) return cuda_fail(e, "prefix kernel");
-    if (p->fwd_staged)
-        e = launch_proj_staged(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_sgroups, p->fwd_slots, p->g, p->d_views,
-                               p->d_xs, p->d_ampv, p->d_xstate, d_proj, proj_dtype, view_begin, view_stride,
-                               view_count, p->margin, p->d_err, st);
+    const int m = method == CTSIM_PROJ_DD ? kDD : kTF;
+    if (p->fwd_staged && p->fwd_columns)
+        e = launch_proj_staged(m, p->fwd_sgroups, staged_slots(p), p->g, p->d_views, p->d_xs, p->d_ampv, p->d_xstate,
+                               d_proj, proj_dtype, view_begin, view_stride, view_count, p->margin, p->d_err, st);
+    else if (p->fwd_staged)
+        e = launch_proj_sums(m, p->fwd_groups, p->fwd_rows, p->fwd_slots, p->g, p->d_views, p->d_xs, p->d_ampv,
+                             p->d_map, d_proj, proj_dtype, view_begin, view_stride, view_count, p->margin, p->d_err,
+                             st);
     else
-        e = launch_proj(method == CTSIM_PROJ_DD ? kDD : kTF, p->fwd_groups, p->fwd_rows, p->fwd_pairs, p->g,
+        e = launch_proj(m, p->fwd_groups, p->fwd_rows, p->fwd_pairs, p->g,
                         p->d_views, p->d_xs, p->d_ampv, p->d_map, d_proj, proj_dtype, view_begin, view_stride,
                         view_count, p->margin, st);
     if (e != cudaSuccess) return cuda_fail(e, "forward projection kernel");
@@ -1161,7 +1187,7 @@ extern "C" bool ctsim_cbct_geom(const char *type, CTSIM_GEOM_PARAMS, const float
 // ---------------------------------------------------------------------------
 extern "C" ctsim_status ctsim_plan_get_tuning(const ctsim_plan *p, ctsim_tuning *t) {
     if (!p || !t) return fail(CTSIM_ERR_ARGUMENT, "null argument");
-    t->proj_groups = p->fwd_staged ? p->fwd_sgroups : p->fwd_groups;
+    t->proj_groups = p->fwd_staged && p->fwd_columns ? p->fwd_sgroups : p->fwd_groups;
     t->proj_rows = p->fwd_rows;
     t->proj_layout = p->fwd_pairs ? 2 : p->fwd_staged ? 3 : 1;
     t->proj_slots = p->fwd_slots;
@@ -1192,11 +1218,16 @@ extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning 
                     "proj_layout must be 1 (sums), 2 (pairs, on a plan whose volume fits them) or 3 (staged columns)");
     {
         const bool staged = t->proj_layout ? t->proj_layout == 3 : p->fwd_staged;
-        const int G = t->proj_groups ? t->proj_groups : p->fwd_sgroups;
-        const int S = t->proj_slots ? t->proj_slots : p->fwd_slots;
         if (t->proj_slots && !proj_slots_valid(p->g.xstride, t->proj_slots))
             return fail(CTSIM_ERR_ARGUMENT, "proj_slots must be 1 .. 64 with slots * column bytes < 1 MiB");
-        if (staged && proj_staged_smem_bytes(p->geom.nv, std::max(p->geom.nx, p->geom.ny), p->g.xstride, G, S) > 200 * 1024)
+        ctsim_plan q = *p;  // as it would be
+        if (t->proj_groups) q.fwd_groups = q.fwd_sgroups = t->proj_groups;
+        if (t->proj_rows) q.fwd_rows = t->proj_rows;
+        if (t->proj_slots) q.fwd_slots = t->proj_slots;
+        // of voxel columns as many as fit are staged, two stages of those asked for at least
+        const bool fits = q.fwd_columns ? staged_fits(&q, 1) && 8LL * q.fwd_slots * column_stride(p->g.nz, 1, 1) <= 200 * 1024
+                                        : staged_fits(&q, q.fwd_slots);
+        if (staged && !fits)
             return fail(CTSIM_ERR_ARGUMENT, "the staged forward projector's shared memory exceeds 200 KiB: fewer slots");
     }
     if (t->proj_groups) p->fwd_groups = p->fwd_sgroups = t->proj_groups;
@@ -1247,14 +1278,23 @@ static std::vector<ctsim_tuning> tuning_candidates(const ctsim_plan *p, int meth
                         ctsim_tuning t = {Gr, 0, 0, 0, R, lay, 0};
                         out.push_back(t);
                     }
-        // staged (proj_rows does not matter to it: the smallest value is valid with every group count)
-        for (int Gr : {1, 2, 4, 8})
-            for (int S : {8, 16, 32})
-                if (proj_slots_valid(p->g.xstride, S) &&
-                    proj_staged_smem_bytes(G.nv, std::max(G.nx, G.ny), p->g.xstride, Gr, S) <= 200 * 1024) {
+        for (int S : {8, 16, 32}) {
+            if (!proj_slots_valid(p->g.xstride, S)) continue;
+            for (int Gr : {1, 2, 4, 8}) {
+                ctsim_plan q = *p;
+                q.fwd_groups = q.fwd_sgroups = Gr;
+                if (p->fwd_columns) {  // proj_rows does not matter: the smallest is valid with every group count
                     ctsim_tuning t = {Gr, 0, 0, 0, 32, 3, S};
-                    out.push_back(t);
+                    if (staged_fits(&q, S)) out.push_back(t);
+                    continue;
                 }
+                for (int R : rows) {
+                    ctsim_tuning t = {Gr, 0, 0, 0, R, 3, S};
+                    q.fwd_rows = R;
+                    if (proj_shape_valid(G.nv, Gr, R) && staged_fits(&q, S)) out.push_back(t);
+                }
+            }
+        }
         return out;
     }
     for (int mz : {1, 2, 4, 8}) {
@@ -1388,22 +1428,25 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
         if ((e = prepare_image(items[i].plan, items[i].in, items[i].in_dtype, st)) != cudaSuccess)
             return cuda_fail(e, "prefix kernel");
     // one persistent launch per launch-shape class: unstaged (0 plain or 1 pairs; row threads,
-    // groups, FP32 out) or staged (2; row pairs per warp, warps, groups, blocks along the
-    // rows, slots, taps, column stride)
+    // groups, FP32 out), staged prefix columns (2; the same and slots) or staged voxel columns (3;
+    // row pairs per warp, warps, groups, blocks along the rows, slots, taps, column stride)
     const int m = method == CTSIM_PROJ_DD ? kDD : kTF;
     std::map<std::vector<int>, std::vector<int>> classes;
     for (int i = 0; i < n; i++) {
         const ctsim_plan *p = items[i].plan;
-        if (p->fwd_staged) {
+        const int lowp = items[i].out_dtype == CTSIM_F32 ? 0 : 1;
+        if (p->fwd_staged && p->fwd_columns) {
             const StagedShape S = staged_shape(p->geom.nv, p->fwd_sgroups);
-            classes[{2, S.np, S.warps, S.parts, S.groups, S.split, p->fwd_slots, p->g.taps, p->g.xstride}].push_back(i);
+            classes[{3, S.np, S.warps, S.parts, S.groups, S.split, staged_slots(p), p->g.taps, p->g.xstride}].push_back(i);
+        } else if (p->fwd_staged) {
+            classes[{2, p->fwd_rows, p->fwd_groups, lowp, p->fwd_slots}].push_back(i);
         } else {
-            classes[{p->fwd_pairs ? 1 : 0, p->fwd_rows, p->fwd_groups, items[i].out_dtype == CTSIM_F32 ? 0 : 1}].push_back(i);
+            classes[{p->fwd_pairs ? 1 : 0, p->fwd_rows, p->fwd_groups, lowp}].push_back(i);
         }
     }
     for (auto &cl : classes) {
         const std::vector<int> &key = cl.first, &idx = cl.second;
-        const bool staged = key[0] == 2;
+        const bool staged = key[0] == 3;
         for (size_t c0 = 0; c0 < idx.size(); c0 += kBatchMax) {
             ProjBatch b;
             b.n = 0;
@@ -1432,12 +1475,13 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
                 T.err = p->d_err;
                 b.total += T.gx * it.view_count * (staged ? key[5] : 1);
                 nlines = std::max(nlines, std::max(p->g.nx, p->g.ny));
-                smem = std::max(smem, staged ? proj_staged_smem_bytes(p->g.nv, nlines, p->g.xstride, p->fwd_sgroups,
-                                                                      p->fwd_slots)
-                                             : proj_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->fwd_groups, p->fwd_rows));
+                smem = std::max(smem, staged ? proj_staged_smem_bytes(p->g.nv, nlines, p->g.xstride, p->fwd_sgroups, key[6])
+                                      : key[0] == 2 ? staged_bytes(p, key[4])
+                                                    : proj_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->fwd_groups, p->fwd_rows));
             }
             e = staged ? launch_proj_staged_batch(m, StagedShape{key[1], key[2], key[3], key[4], key[5]}, key[7], key[6], nlines, smem,
                                                   b, st)
+                : key[0] == 2 ? launch_proj_sums_batch(m, key[2], key[1], key[4], key[3] != 0, smem, b, st)
                        : launch_proj_batch(m, key[2], key[1], key[0] == 1, key[3] != 0, smem, b, st);
             if (e != cudaSuccess) return cuda_fail(e, "batched forward projection");
         }

@@ -57,9 +57,10 @@ struct Geom {
     int xpad, taps;               // staged columns: zeros below voxel 0; voxels that a detector row can reach
 };
 
-// Column stride of the plain prefix sums (X[0..nz] and X[nz] repeated above it) and of the
-// staged columns (xpad zeros, nz voxels, `taps` zeros), rounded up to 4 floats so that every
-// column starts on a 16-byte boundary (the bulk copies need that).  xpad >= 1, taps >= 2.
+// Column stride of the staged columns (xpad zeros, nz voxels, `taps` zeros; xpad >= 1, taps >=
+// 2), rounded up to 4 floats so that every column starts on a 16-byte boundary (the bulk copies
+// need that); with xpad = taps = 1 that of the plain prefix sums (X[0..nz] and at least one copy
+// of X[nz] above it).
 __host__ __device__ inline int column_stride(int nz, int xpad, int taps) { return (nz + xpad + taps + 3) & ~3; }
 
 // Per-view constants, geom/cbct/cbct_proj.c:256-265 and cbct_back.c:50-52.

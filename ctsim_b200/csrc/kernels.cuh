@@ -80,6 +80,13 @@ struct StagedShape {
 StagedShape staged_shape(int nv, int groups);
 int staged_columns(const StagedShape &shape, int nu);
 
+// The same with the candidates' prefix columns (launch_prefix, single sums) staged in two
+// buffers of `slots` columns (proj_sums.cu); groups and rows as launch_proj.
+cudaError_t launch_proj_sums(int method, int groups, int rows, int slots, const Geom &g, const View *views,
+                             const float *xs, const float *ampv, const uint8_t *map, void *proj, int out_dtype,
+                             int view_begin, int view_stride, int view_count, float margin, int *err, cudaStream_t st);
+size_t proj_sums_smem_bytes(int nv, int nx, int ny, int xstride, int groups, int rows, int slots);
+
 // voxel-driven bilinear modes: back,pd (v outside the detector skipped), back,hpd (v
 // clamped), back,var (geom/cbct/cbct_back_var.c)
 enum PdMode { kPdOff = 0, kPdClamp = 1, kPdVar = 2 };
@@ -141,6 +148,9 @@ cudaError_t launch_back_batch(int method, int mz, bool vec, bool lowp, size_t sm
 // column stride; nlines: the largest max(nx, ny).
 cudaError_t launch_proj_staged_batch(int method, const StagedShape &shape, int taps, int slots, int nlines, size_t smem,
                                      const ProjBatch &b, cudaStream_t st);
+// proj_sums.cu over a batch of plans of one group count, row threads and slots.
+cudaError_t launch_proj_sums_batch(int method, int groups, int row_threads, int slots, bool lowp, size_t smem,
+                                   const ProjBatch &b, cudaStream_t st);
 // Blocks of a persistent launch: the resident blocks of the device, at most `total`.
 int persistent_grid(const void *kernel, int threads, size_t smem, int total);
 

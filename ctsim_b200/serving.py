@@ -88,11 +88,9 @@ def hbm_footprint(req: ReconRequest) -> int:
     L = 64
     while L < 2 * g.nu - 1:
         L *= 2
-    # the forward projector's form of the image: paired prefix sums or padded voxel columns
-    # (zeros for the voxels that a detector row can reach past either end) at most
-    reach = g.detSpacing[1] / g.reconSpacing[2] * (g.SAD + math.hypot(g.nx * g.reconSpacing[0], g.ny *
-                                                                      g.reconSpacing[1])) / g.SDD
-    xs = 4 * g.nx * g.ny * max(2 * (g.nz + 4), g.nz + 2 * int(reach + 1) + 8)
+    # the forward projector's form of the image: paired prefix sums or voxel columns padded for
+    # rows of up to eight voxels, at most
+    xs = 4 * g.nx * g.ny * max(2 * (g.nz + 4), g.nz + 20)
     plan = xs + 4 * g.nu * g.nv + 2 * g.nx * g.ny + 64 * g.noViews + 4096
     fdk = s * pix + 4 * g.nu * g.nv + 12 * L + 4 * g.nu * g.noViews + 4096  # filtered sinogram + tables
     image = 4 * vox
