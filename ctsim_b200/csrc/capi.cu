@@ -59,7 +59,7 @@ int pow2_at_least(int v) {
 
 struct ctsim_plan {
     ctsim_geom geom{};
-    Geom g{};
+    ColumnsGeom g{};
     int device = 0;
     View *d_views = nullptr;
     float *d_ampv = nullptr;
@@ -238,7 +238,7 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     p->stream_ordered = stream_ordered;
     p->stream = stream;
     p->betas.assign(betas, betas + G.noviews);
-    Geom &g = p->g;
+    ColumnsGeom &g = p->g;
     g.nx = G.nx; g.ny = G.ny; g.nz = G.nz; g.nu = G.nu; g.nv = G.nv; g.det = G.detector_type;
     g.dx = G.dx; g.dy = G.dy; g.dz = G.dz; g.sad = G.sad; g.sdd = G.sdd; g.du = G.du; g.dv = G.dv;
     g.wx = centre(G.nx, G.offset_x);

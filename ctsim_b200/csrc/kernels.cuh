@@ -67,9 +67,10 @@ size_t proj_smem_bytes(int nv, int nx, int ny, int groups, int rows);
 // of *err.
 cudaError_t launch_columns(const void *image, int in_dtype, const uint8_t *map, float *xs, uint8_t *state, int nxy,
                            int nz, int xpad, int xstride, cudaStream_t st);
-cudaError_t launch_proj_staged(int method, int groups, int slots, const Geom &g, const View *views, const float *xs,
-                               const float *ampv, const uint8_t *state, void *proj, int out_dtype, int view_begin,
-                               int view_stride, int view_count, float margin, int *err, cudaStream_t st);
+cudaError_t launch_proj_staged(int method, int groups, int slots, const ColumnsGeom &g, const View *views,
+                               const float *xs, const float *ampv, const uint8_t *state, void *proj, int out_dtype,
+                               int view_begin, int view_stride, int view_count, float margin, int *err,
+                               cudaStream_t st);
 size_t proj_staged_smem_bytes(int nv, int nlines, int xstride, int groups, int slots);
 bool proj_slots_valid(int xstride, int slots);
 // Row pairs per consumer warp; consumer warps along the rows, the columns and the
@@ -103,7 +104,7 @@ cudaError_t launch_pd(int mode, int mz, const Geom &g, const View *views, const 
 constexpr int kBatchMax = 64;  // tasks per launch (the task table travels as a kernel parameter)
 
 struct ProjTask {
-    Geom g;
+    ColumnsGeom g;
     const View *views;
     const float *xs;
     const float *ampv;

@@ -331,7 +331,7 @@ __device__ __forceinline__ void staged_weights(const ColumnFP &fp, float scl, fl
 // One work item: detector columns from bx kPart parts on of launch view by, row pairs from
 // bz PB on (PB: row pairs of a block).
 struct StagedItem {
-    const Geom *g;
+    const ColumnsGeom *g;
     const View *views;
     const float *xs, *ampv;
     const uint8_t *state;  // of the columns (columns_kernel)
@@ -350,7 +350,7 @@ struct StagedView {
     // pair q covers rows [mid - 32 (q + 1), mid - 32 q) and [mid + 32 q, mid + 32 (q + 1)); all
     // pairs together cover the detector wherever mid is clamped to
     __device__ __forceinline__ StagedView(const StagedItem &I, int parts, int PB) {
-        const Geom &g = *I.g;
+        const ColumnsGeom &g = *I.g;
         v = I.views[I.view_begin + I.by * I.view_stride];
         iu0 = I.bx * kPart * parts;
         const int half = 32 * ((g.nv + 63) / 64);
@@ -367,7 +367,7 @@ struct StagedView {
 template <int METHOD>
 __device__ __forceinline__ bool staged_produce(const StagedItem &I, const StagedSmem &L, StagedRing *ring, RingPos &at,
                                                int PB) {
-    const Geom &g = *I.g;
+    const ColumnsGeom &g = *I.g;
     char *smem = reinterpret_cast<char *>(ring) + L.ring_bytes();
     float *columns = reinterpret_cast<float *>(smem);  // [kRing][slots][xstride]
     char *entries = smem + L.column_bytes() + L.sum_bytes();
@@ -494,7 +494,7 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
 template <int NP, int TAPS>
 __device__ __forceinline__ bool staged_consume(const StagedItem &I, const StagedSmem &L, StagedRing *ring, RingPos &at,
                                                int wg, int consumers) {
-    const Geom &g = *I.g;
+    const ColumnsGeom &g = *I.g;
     char *smem = reinterpret_cast<char *>(ring) + L.ring_bytes();
     float *sum = reinterpret_cast<float *>(smem + L.column_bytes());  // [columns][pairs][2][32]
     // [kRing][parts][entries]: {pa, pb, 1 / zinc, column address}, four weights, each twice
@@ -642,8 +642,9 @@ __device__ __forceinline__ void staged_block(int total, int groups, int parts, i
 
 template <int METHOD, int NP, int CW, int TAPS>
 __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * StagedRegs<NP, CW>::kLaunch))
-    proj_staged_kernel(const __grid_constant__ Geom g, const View *__restrict__ views, const float *__restrict__ xs,
-                       const float *__restrict__ ampv, const uint8_t *__restrict__ state, void *__restrict__ proj,
+    proj_staged_kernel(const __grid_constant__ ColumnsGeom g, const View *__restrict__ views,
+                       const float *__restrict__ xs, const float *__restrict__ ampv,
+                       const uint8_t *__restrict__ state, void *__restrict__ proj,
                        int out_dtype, int view_begin, int view_stride, float margin, int groups, int parts,
                        int slots, int *__restrict__ err, int ngx, int vc, int total) {
     staged_block<METHOD, NP, CW, TAPS>(total, groups, parts, slots, max(g.nx, g.ny), [&](int blk) {
@@ -714,9 +715,9 @@ bool proj_slots_valid(int xstride, int slots) {
         return cudaGetLastError();                                               \
     }
 
-cudaError_t launch_proj_staged(int method, int groups, int slots, const Geom &g, const View *views, const float *xs,
-                               const float *ampv, const uint8_t *state, void *proj, int out_dtype, int vb, int vs,
-                               int vc, float margin, int *err, cudaStream_t st) {
+cudaError_t launch_proj_staged(int method, int groups, int slots, const ColumnsGeom &g, const View *views,
+                               const float *xs, const float *ampv, const uint8_t *state, void *proj, int out_dtype,
+                               int vb, int vs, int vc, float margin, int *err, cudaStream_t st) {
     if ((groups != 1 && groups != 2 && groups != 4 && groups != 8) || !proj_slots_valid(g.xstride, slots) ||
         g.xstride % 4 != 0 || g.xpad < 1 || g.taps < 2 || g.xstride < g.nz + g.xpad + g.taps ||
         reinterpret_cast<uintptr_t>(xs) % 16 != 0)
