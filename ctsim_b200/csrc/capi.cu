@@ -1230,13 +1230,14 @@ extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning 
         if (staged && !fits)
             return fail(CTSIM_ERR_ARGUMENT, "the staged forward projector's shared memory exceeds 200 KiB: fewer slots");
     }
-    if (t->proj_groups) p->fwd_groups = p->fwd_sgroups = t->proj_groups;
-    if (t->proj_rows) p->fwd_rows = t->proj_rows;
-    if (t->proj_slots) p->fwd_slots = t->proj_slots;
     if (t->proj_layout) {
         p->fwd_pairs = t->proj_layout == 2;
         p->fwd_staged = t->proj_layout == 3;
     }
+    // the group count of the projector that now runs; the other one keeps its own
+    if (t->proj_groups) (p->fwd_staged && p->fwd_columns ? p->fwd_sgroups : p->fwd_groups) = t->proj_groups;
+    if (t->proj_rows) p->fwd_rows = t->proj_rows;
+    if (t->proj_slots) p->fwd_slots = t->proj_slots;
     if (t->back_mz) {
         p->back_mz = t->back_mz;
         p->back_qcap = back_qcap_for(p, t->back_mz);
@@ -1247,6 +1248,21 @@ extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning 
     }
     if (t->pd_mz) p->pd_mz = t->pd_mz;
     return CTSIM_OK;
+}
+
+// Every launch shape of `from`, both projectors' group counts among them (ctsim_tuning has one).
+static void restore_tuning(ctsim_plan *p, const ctsim_plan &from) {
+    p->fwd_groups = from.fwd_groups;
+    p->fwd_sgroups = from.fwd_sgroups;
+    p->fwd_rows = from.fwd_rows;
+    p->fwd_pairs = from.fwd_pairs;
+    p->fwd_staged = from.fwd_staged;
+    p->fwd_slots = from.fwd_slots;
+    p->back_mz = from.back_mz;
+    p->back_qcap = from.back_qcap;
+    p->back_mz_tf = from.back_mz_tf;
+    p->back_qcap_tf = from.back_qcap_tf;
+    p->pd_mz = from.pd_mz;
 }
 
 namespace {
@@ -1345,8 +1361,7 @@ extern "C" ctsim_status ctsim_plan_autotune(ctsim_plan *p, int method, int sampl
             ctsim_plan_release(p, img);
             return fail(CTSIM_ERR_ALLOC, std::string("autotune buffers: ") + cudaGetErrorString(e));
         }
-        ctsim_tuning saved;
-        ctsim_plan_get_tuning(p, &saved);
+        const ctsim_plan saved = *p;
         float best_ms = 0.f;
         ctsim_status s = CTSIM_OK;
         if ((e = cudaMemsetAsync(img, 0, nimg * 4, st)) != cudaSuccess ||
@@ -1382,7 +1397,7 @@ extern "C" ctsim_status ctsim_plan_autotune(ctsim_plan *p, int method, int sampl
         if (e1) cudaEventDestroy(e1);
         ctsim_plan_release(p, img);
         ctsim_plan_release(p, sino);
-        ctsim_plan_set_tuning(p, &saved);
+        restore_tuning(p, saved);
         if (s != CTSIM_OK) return s;
         if (!have) return fail(CTSIM_ERR_UNSUPPORTED, "no valid launch shape");
         std::lock_guard<std::mutex> lock(g_tune_mutex);

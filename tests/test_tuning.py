@@ -1,0 +1,52 @@
+"""Launch shapes that are set, restored, tuned and reused: what one method's tuning leaves to the
+others, detectors too tall for some shapes, plans of the same sizes and other spacings."""
+import time
+
+import numpy as np
+import pytest
+
+from ctsim_b200 import CTGeometry, circular_betas
+
+pytestmark = pytest.mark.gpu
+
+
+def _geom(nz=30, nv=160, dz=1.0, dv=0.5, n=14, views=7, nu=36):
+    return CTGeometry((n, n - 2, nz), (1.0, 1.0, dz), (0.3, 0, 0), (nu, nv), (1.6, dv), (0, 0), 1000.0, 500.0, 1500.0,
+                      circular_betas(views))
+
+
+def _image(g):
+    import torch
+    return torch.from_numpy(np.random.default_rng(3).random(g.image_shape, dtype=np.float32)).cuda()
+
+
+def test_tuning_one_method_leaves_the_forward_projectors_as_they_were():
+    import torch
+    from ctsim_b200.projector import Plan
+    g = _geom()
+    x = _image(g)
+    fresh, tuned = Plan(g), Plan(g)
+    assert fresh.tuning["proj_layout"] == 3
+    tuned.autotune("back,dd", 3)
+    tuned.autotune("back,hpd", 3)
+    for layout in (2, 1, 3):
+        fresh.set_tuning(proj_layout=layout)
+        tuned.set_tuning(proj_layout=layout)
+        assert {k: fresh.tuning[k] for k in ("proj_groups", "proj_rows", "proj_slots")} == {
+            k: tuned.tuning[k] for k in ("proj_groups", "proj_rows", "proj_slots")}
+        assert torch.equal(fresh.project(x, "dd"), tuned.project(x, "dd")), layout
+
+
+def test_set_tuning_takes_back_what_get_tuning_gave():
+    import torch
+    from ctsim_b200.projector import Plan
+    g = _geom()
+    x = _image(g)
+    plan = Plan(g)
+    for layout, groups in ((3, 4), (2, 8), (1, 1)):
+        plan.set_tuning(proj_layout=layout, proj_groups=groups, proj_rows=32)
+        want, saved = plan.project(x, "dd"), plan.tuning
+        other = Plan(g)
+        other.set_tuning(**saved)
+        assert other.tuning == saved
+        assert torch.equal(other.project(x, "dd"), want), layout
