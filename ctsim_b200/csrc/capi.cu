@@ -1199,57 +1199,6 @@ extern "C" ctsim_status ctsim_plan_get_tuning(const ctsim_plan *p, ctsim_tuning 
 
 static bool mz_valid(int mz) { return mz == 1 || mz == 2 || mz == 4 || mz == 8; }
 
-extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning *t) {
-    if (!p || !t) return fail(CTSIM_ERR_ARGUMENT, "null argument");
-    if (t->proj_groups || t->proj_rows) {
-        const int G = t->proj_groups ? t->proj_groups : p->fwd_groups;
-        const int R = t->proj_rows ? t->proj_rows : p->fwd_rows;
-        if (!proj_shape_valid(p->geom.nv, G, R) || proj_smem_bytes(p->geom.nv, p->geom.nx, p->geom.ny, G, R) > 200 * 1024)
-            return fail(CTSIM_ERR_ARGUMENT,
-                        "proj_groups must be 1, 2, 4 or 8 and proj_rows a multiple of 32 up to the rows' need, "
-                        "with groups * rows <= 256");
-    }
-    if ((t->back_mz && (!mz_valid(t->back_mz) || !back_mz_fits(p, t->back_mz))) ||
-        (t->back_mz_tf && (!mz_valid(t->back_mz_tf) || !back_mz_fits(p, t->back_mz_tf))))
-        return fail(CTSIM_ERR_ARGUMENT, "back_mz must be 1, 2, 4 or 8 and fit the row buffer");
-    if (t->pd_mz && !mz_valid(t->pd_mz)) return fail(CTSIM_ERR_ARGUMENT, "pd_mz must be 1, 2, 4 or 8");
-    if (t->proj_layout && t->proj_layout != 1 && t->proj_layout != 3 && !(t->proj_layout == 2 && p->xs_holds_pairs))
-        return fail(CTSIM_ERR_ARGUMENT,
-                    "proj_layout must be 1 (sums), 2 (pairs, on a plan whose volume fits them) or 3 (staged columns)");
-    {
-        const bool staged = t->proj_layout ? t->proj_layout == 3 : p->fwd_staged;
-        if (t->proj_slots && !proj_slots_valid(p->g.xstride, t->proj_slots))
-            return fail(CTSIM_ERR_ARGUMENT, "proj_slots must be 1 .. 64 with slots * column bytes < 1 MiB");
-        ctsim_plan q = *p;  // as it would be
-        if (t->proj_groups) q.fwd_groups = q.fwd_sgroups = t->proj_groups;
-        if (t->proj_rows) q.fwd_rows = t->proj_rows;
-        if (t->proj_slots) q.fwd_slots = t->proj_slots;
-        // of voxel columns as many as fit are staged, two stages of those asked for at least
-        const bool fits = q.fwd_columns ? staged_fits(&q, 1) && 8LL * q.fwd_slots * column_stride(p->g.nz, 1, 1) <= 200 * 1024
-                                        : staged_fits(&q, q.fwd_slots);
-        if (staged && !fits)
-            return fail(CTSIM_ERR_ARGUMENT, "the staged forward projector's shared memory exceeds 200 KiB: fewer slots");
-    }
-    if (t->proj_layout) {
-        p->fwd_pairs = t->proj_layout == 2;
-        p->fwd_staged = t->proj_layout == 3;
-    }
-    // the group count of the projector that now runs; the other one keeps its own
-    if (t->proj_groups) (p->fwd_staged && p->fwd_columns ? p->fwd_sgroups : p->fwd_groups) = t->proj_groups;
-    if (t->proj_rows) p->fwd_rows = t->proj_rows;
-    if (t->proj_slots) p->fwd_slots = t->proj_slots;
-    if (t->back_mz) {
-        p->back_mz = t->back_mz;
-        p->back_qcap = back_qcap_for(p, t->back_mz);
-    }
-    if (t->back_mz_tf) {
-        p->back_mz_tf = t->back_mz_tf;
-        p->back_qcap_tf = back_qcap_for(p, t->back_mz_tf);
-    }
-    if (t->pd_mz) p->pd_mz = t->pd_mz;
-    return CTSIM_OK;
-}
-
 // Every launch shape of `from`, both projectors' group counts among them (ctsim_tuning has one).
 static void restore_tuning(ctsim_plan *p, const ctsim_plan &from) {
     p->fwd_groups = from.fwd_groups;
@@ -1263,6 +1212,56 @@ static void restore_tuning(ctsim_plan *p, const ctsim_plan &from) {
     p->back_mz_tf = from.back_mz_tf;
     p->back_qcap_tf = from.back_qcap_tf;
     p->pd_mz = from.pd_mz;
+}
+
+extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning *t) {
+    if (!p || !t) return fail(CTSIM_ERR_ARGUMENT, "null argument");
+    if ((t->back_mz && (!mz_valid(t->back_mz) || !back_mz_fits(p, t->back_mz))) ||
+        (t->back_mz_tf && (!mz_valid(t->back_mz_tf) || !back_mz_fits(p, t->back_mz_tf))))
+        return fail(CTSIM_ERR_ARGUMENT, "back_mz must be 1, 2, 4 or 8 and fit the row buffer");
+    if (t->pd_mz && !mz_valid(t->pd_mz)) return fail(CTSIM_ERR_ARGUMENT, "pd_mz must be 1, 2, 4 or 8");
+    if (t->proj_layout && t->proj_layout != 1 && t->proj_layout != 3 && !(t->proj_layout == 2 && p->xs_holds_pairs))
+        return fail(CTSIM_ERR_ARGUMENT,
+                    "proj_layout must be 1 (sums), 2 (pairs, on a plan whose volume fits them) or 3 (staged columns)");
+    if (t->proj_slots && !proj_slots_valid(p->g.xstride, t->proj_slots))
+        return fail(CTSIM_ERR_ARGUMENT, "proj_slots must be 1 .. 64 with slots * column bytes < 1 MiB");
+    if (t->proj_groups || t->proj_rows || t->proj_layout || t->proj_slots) {
+        const ctsim_geom &G = p->geom;
+        ctsim_plan q = *p;  // the forward projector as it would be
+        if (t->proj_layout) {
+            q.fwd_pairs = t->proj_layout == 2;
+            q.fwd_staged = t->proj_layout == 3;
+        }
+        const bool columns = q.fwd_staged && q.fwd_columns;
+        // the group count of the projector that runs then; the other one keeps its own
+        if (t->proj_groups) (columns ? q.fwd_sgroups : q.fwd_groups) = t->proj_groups;
+        if (t->proj_rows) q.fwd_rows = t->proj_rows;
+        if (t->proj_slots) q.fwd_slots = t->proj_slots;
+        // staged voxel columns take every group count and no row threads (any that one group may have)
+        const int S = q.fwd_sgroups;
+        if (columns ? (S != 1 && S != 2 && S != 4 && S != 8) || !proj_shape_valid(G.nv, 1, q.fwd_rows)
+                    : !proj_shape_valid(G.nv, q.fwd_groups, q.fwd_rows) ||
+                          proj_smem_bytes(G.nv, G.nx, G.ny, q.fwd_groups, q.fwd_rows) > 200 * 1024)
+            return fail(CTSIM_ERR_ARGUMENT,
+                        "proj_groups must be 1, 2, 4 or 8 and proj_rows a multiple of 32 up to the rows' need, "
+                        "with groups * rows <= 256");
+        // of voxel columns as many as fit are staged, two stages of those asked for at least
+        const bool fits = columns ? staged_fits(&q, 1) && 8LL * q.fwd_slots * column_stride(G.nz, 1, 1) <= 200 * 1024
+                                  : !q.fwd_staged || staged_fits(&q, q.fwd_slots);
+        if (!fits)
+            return fail(CTSIM_ERR_ARGUMENT, "the staged forward projector's shared memory exceeds 200 KiB: fewer slots");
+        restore_tuning(p, q);
+    }
+    if (t->back_mz) {
+        p->back_mz = t->back_mz;
+        p->back_qcap = back_qcap_for(p, t->back_mz);
+    }
+    if (t->back_mz_tf) {
+        p->back_mz_tf = t->back_mz_tf;
+        p->back_qcap_tf = back_qcap_for(p, t->back_mz_tf);
+    }
+    if (t->pd_mz) p->pd_mz = t->pd_mz;
+    return CTSIM_OK;
 }
 
 namespace {
@@ -1299,7 +1298,7 @@ static std::vector<ctsim_tuning> tuning_candidates(const ctsim_plan *p, int meth
             for (int Gr : {1, 2, 4, 8}) {
                 ctsim_plan q = *p;
                 q.fwd_groups = q.fwd_sgroups = Gr;
-                if (p->fwd_columns) {  // proj_rows does not matter: the smallest is valid with every group count
+                if (p->fwd_columns) {  // proj_rows does not matter
                     ctsim_tuning t = {Gr, 0, 0, 0, 32, 3, S};
                     if (staged_fits(&q, S)) out.push_back(t);
                     continue;
@@ -1370,7 +1369,7 @@ extern "C" ctsim_status ctsim_plan_autotune(ctsim_plan *p, int method, int sampl
             s = cuda_fail(e, "autotune set-up");
         }
         for (size_t i = 0; s == CTSIM_OK && i < cand.size(); i++) {
-            if ((s = ctsim_plan_set_tuning(p, &cand[i])) != CTSIM_OK) break;
+            if (ctsim_plan_set_tuning(p, &cand[i]) != CTSIM_OK) continue;  // a shape this plan does not take
             float ms = 0.f;
             for (int rep = 0; rep < 3 && s == CTSIM_OK; rep++) {  // one warm-up, then the faster of two
                 cudaEventRecord(e0, st);

@@ -50,3 +50,31 @@ def test_set_tuning_takes_back_what_get_tuning_gave():
         other.set_tuning(**saved)
         assert other.tuning == saved
         assert torch.equal(other.project(x, "dd"), want), layout
+
+
+@pytest.mark.parametrize("nv,dv", [(768, 0.5), (1100, 0.4), (768, 4.0)])
+def test_autotune_and_groups_on_tall_detectors(nv, dv):
+    """Detectors of which the unstaged projector's shared memory does not hold eight groups."""
+    import torch
+    from ctsim_b200._lib import CtsimError
+    from ctsim_b200.projector import Plan
+    from oracle.bindings import oracle_cbct
+    g = _geom(nz=90, nv=nv, dv=dv)
+    x = _image(g)
+    want = {m: oracle_cbct(f"proj,{m}", g, x.cpu().numpy()) for m in ("dd", "tf")}
+    plan = Plan(g)
+    assert plan.tuning["proj_layout"] == 3
+    for groups in (1, 2, 4, 8):
+        plan.set_tuning(proj_groups=groups, proj_rows=32, proj_layout=3)
+        for m in ("dd", "tf"):
+            got = plan.project(x, m).cpu().numpy()
+            assert np.linalg.norm(got - want[m]) <= 1e-5 * np.linalg.norm(want[m]), (groups, m)
+    with pytest.raises(CtsimError):
+        plan.set_tuning(proj_groups=8, proj_rows=32, proj_layout=1)
+    with pytest.raises(CtsimError):
+        plan.set_tuning(proj_groups=3, proj_layout=3)
+    for m in ("dd", "tf"):
+        t = plan.autotune(f"proj,{m}", 2)
+        assert t["proj_layout"] in (1, 2, 3)
+        got = plan.project(x, m).cpu().numpy()
+        assert np.linalg.norm(got - want[m]) <= 1e-5 * np.linalg.norm(want[m]), m
