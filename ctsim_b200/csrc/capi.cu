@@ -1266,7 +1266,7 @@ extern "C" ctsim_status ctsim_plan_set_tuning(ctsim_plan *p, const ctsim_tuning 
 
 namespace {
 // Choices measured in this process, by shape class: method, the volume and detector
-// sizes and the detector type.
+// sizes, the detector type and what the method's launch shapes take from the spacings.
 std::mutex g_tune_mutex;
 std::map<std::vector<int>, ctsim_tuning> g_tuned;
 }  // namespace
@@ -1331,7 +1331,10 @@ extern "C" ctsim_status ctsim_plan_autotune(ctsim_plan *p, int method, int sampl
     if ((fwd || !vox) && !p->fwd_ok) return fail(CTSIM_ERR_UNSUPPORTED, p->fwd_reason);
     if (p->g.det == 2 && method != CTSIM_PROJ_DD && method != CTSIM_BACK_DD) return fail(CTSIM_ERR_UNSUPPORTED, kArcOnlyDD);
     const ctsim_geom &G = p->geom;
-    const std::vector<int> key = {method, G.nx, G.ny, G.nz, G.nu, G.nv, G.detector_type};
+    std::vector<int> key = {method, G.nx, G.ny, G.nz, G.nu, G.nv, G.detector_type};
+    // what the spacings decide besides: the voxels of a row and the staged form, or the rows of a voxel
+    if (fwd) key.insert(key.end(), {p->g.taps, p->g.xstride, p->fwd_columns});
+    else if (!vox) key.insert(key.end(), {(int)p->zinc_max, back_qcap_for(p, 1), back_qcap_for(p, 8)});
     bool have = false;
     ctsim_tuning best = {0, 0, 0, 0, 0, 0, 0};
     {
@@ -1339,7 +1342,7 @@ extern "C" ctsim_status ctsim_plan_autotune(ctsim_plan *p, int method, int sampl
         auto it = g_tuned.find(key);
         if (it != g_tuned.end()) {
             best = it->second;
-            have = true;
+            have = ctsim_plan_set_tuning(p, &best) == CTSIM_OK;  // measured again where this plan refuses it
         }
     }
     if (!have) {

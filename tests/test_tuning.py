@@ -78,3 +78,29 @@ def test_autotune_and_groups_on_tall_detectors(nv, dv):
         assert t["proj_layout"] in (1, 2, 3)
         got = plan.project(x, m).cpu().numpy()
         assert np.linalg.norm(got - want[m]) <= 1e-5 * np.linalg.norm(want[m]), m
+
+
+def test_choices_are_kept_by_spacings_too():
+    """A choice is reused for the same geometry, measured anew for plans of the same sizes whose
+    rows or voxels are longer.  Reuse takes microseconds, measuring two dozen shapes of 60 views
+    takes tens of milliseconds."""
+    import torch
+    from ctsim_b200 import _lib
+    from ctsim_b200.projector import Plan
+
+    def seconds(plan, method):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        plan.autotune(method, 60)
+        return time.perf_counter() - t0
+
+    _lib.check(_lib.load().ctsim_autotune_clear())
+    plans = [Plan(_geom(nz=64, nv=90, dv=dv, dz=dz, n=64, views=60, nu=90))
+             for dv, dz in ((1.6, 1.0), (1.6, 1.0), (6.0, 1.0), (20.0, 1.0), (1.6, 4.0))]
+    for method in ("proj,dd", "back,dd"):
+        first, again, long_rows, longer, tall = [seconds(p, method) for p in plans]
+        assert again < 0.1 * first, method
+        if method == "proj,dd":
+            assert long_rows > 10 * again and longer > 10 * again
+        else:
+            assert tall > 10 * again
