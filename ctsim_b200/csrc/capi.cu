@@ -1446,7 +1446,7 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
             return cuda_fail(e, "prefix kernel");
     // one persistent launch per launch-shape class: unstaged (0 plain or 1 pairs; row threads,
     // groups, FP32 out), staged prefix columns (2; the same and slots) or staged voxel columns (3;
-    // row pairs per warp, warps, groups, blocks along the rows, slots, taps, column stride)
+    // row pairs per warp, warps, groups, blocks along the rows, the rows' voxels up to three)
     const int m = method == CTSIM_PROJ_DD ? kDD : kTF;
     std::map<std::vector<int>, std::vector<int>> classes;
     for (int i = 0; i < n; i++) {
@@ -1454,7 +1454,7 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
         const int lowp = items[i].out_dtype == CTSIM_F32 ? 0 : 1;
         if (p->fwd_staged && p->fwd_columns) {
             const StagedShape S = staged_shape(p->geom.nv, p->fwd_sgroups);
-            classes[{3, S.np, S.warps, S.parts, S.groups, S.split, staged_slots(p), p->g.taps, p->g.xstride}].push_back(i);
+            classes[{3, S.np, S.warps, S.parts, S.groups, S.split, p->g.taps <= 3 ? p->g.taps : 0}].push_back(i);
         } else if (p->fwd_staged) {
             classes[{2, p->fwd_rows, p->fwd_groups, lowp, p->fwd_slots}].push_back(i);
         } else {
@@ -1464,12 +1464,13 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
     for (auto &cl : classes) {
         const std::vector<int> &key = cl.first, &idx = cl.second;
         const bool staged = key[0] == 3;
+        const StagedShape shape = staged ? StagedShape{key[1], key[2], key[3], key[4], key[5]} : StagedShape{};
         for (size_t c0 = 0; c0 < idx.size(); c0 += kBatchMax) {
             ProjBatch b;
             b.n = 0;
             b.total = 0;
             size_t smem = 0;
-            int nlines = 1;
+            int nlines = 1, xstride = 0, slots = 64;  // of the class: the largest two, the fewest slots
             for (size_t c = c0; c < std::min(idx.size(), c0 + kBatchMax); c++) {
                 const ctsim_batch_item &it = items[idx[c]];
                 const ctsim_plan *p = it.plan;
@@ -1485,21 +1486,30 @@ extern "C" ctsim_status ctsim_batch_project(int method, const ctsim_batch_item *
                 T.vb = it.view_begin;
                 T.vs = it.view_stride;
                 T.vc = it.view_count;
-                T.gx = staged ? staged_columns(StagedShape{key[1], key[2], key[3], key[4], key[5]}, p->g.nu)
-                              : (p->g.nu + kProjGroupWidth - 1) / kProjGroupWidth;
+                T.gx = staged ? staged_columns(shape, p->g.nu) : (p->g.nu + kProjGroupWidth - 1) / kProjGroupWidth;
                 T.first = b.total;
                 T.margin = p->margin;
                 T.err = p->d_err;
                 b.total += T.gx * it.view_count * (staged ? key[5] : 1);
-                nlines = std::max(nlines, std::max(p->g.nx, p->g.ny));
-                smem = std::max(smem, staged ? proj_staged_smem_bytes(p->g.nv, nlines, p->g.xstride, p->fwd_sgroups, key[6])
-                                      : key[0] == 2 ? staged_bytes(p, key[4])
-                                                    : proj_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->fwd_groups, p->fwd_rows));
+                if (staged) {
+                    nlines = std::max(nlines, std::max(p->g.nx, p->g.ny));
+                    xstride = std::max(xstride, p->g.xstride);
+                    slots = std::min(slots, staged_slots(p));
+                } else {
+                    smem = std::max(smem, key[0] == 2 ? staged_bytes(p, key[4])
+                                                      : proj_smem_bytes(p->g.nv, p->g.nx, p->g.ny, p->fwd_groups,
+                                                                        p->fwd_rows));
+                }
             }
-            e = staged ? launch_proj_staged_batch(m, StagedShape{key[1], key[2], key[3], key[4], key[5]}, key[7], key[6], nlines, smem,
-                                                  b, st)
-                : key[0] == 2 ? launch_proj_sums_batch(m, key[2], key[1], key[4], key[3] != 0, smem, b, st)
-                       : launch_proj_batch(m, key[2], key[1], key[0] == 1, key[3] != 0, smem, b, st);
+            if (staged) {
+                while (slots > 1 && proj_staged_smem_bytes(shape, nlines, xstride, slots) > 200 * 1024) slots--;
+                smem = proj_staged_smem_bytes(shape, nlines, xstride, slots);
+                e = launch_proj_staged_batch(m, shape, key[6], slots, xstride, nlines, smem, b, st);
+            } else if (key[0] == 2) {
+                e = launch_proj_sums_batch(m, key[2], key[1], key[4], key[3] != 0, smem, b, st);
+            } else {
+                e = launch_proj_batch(m, key[2], key[1], key[0] == 1, key[3] != 0, smem, b, st);
+            }
             if (e != cudaSuccess) return cuda_fail(e, "batched forward projection");
         }
     }

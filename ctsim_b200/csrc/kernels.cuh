@@ -145,10 +145,11 @@ cudaError_t launch_proj_batch(int method, int groups, int row_threads, bool pair
                               const ProjBatch &b, cudaStream_t st);
 cudaError_t launch_back_batch(int method, int mz, bool vec, bool lowp, size_t smem, const BackBatch &b,
                               cudaStream_t st, int src = kSrcScaled);
-// The staged forward projector (launch_proj_staged) over a batch of plans of one shape and
-// column stride; nlines: the largest max(nx, ny).
-cudaError_t launch_proj_staged_batch(int method, const StagedShape &shape, int taps, int slots, int nlines, size_t smem,
-                                     const ProjBatch &b, cudaStream_t st);
+// The staged forward projector (launch_proj_staged) over a batch of plans of one shape (and, up to
+// three, of one `taps`); xstride and nlines: the largest column stride and max(nx, ny).
+size_t proj_staged_smem_bytes(const StagedShape &shape, int nlines, int xstride, int slots);
+cudaError_t launch_proj_staged_batch(int method, const StagedShape &shape, int taps, int slots, int xstride, int nlines,
+                                     size_t smem, const ProjBatch &b, cudaStream_t st);
 // proj_sums.cu over a batch of plans of one group count, row threads and slots.
 cudaError_t launch_proj_sums_batch(int method, int groups, int row_threads, int slots, bool lowp, size_t smem,
                                    const ProjBatch &b, cudaStream_t st);

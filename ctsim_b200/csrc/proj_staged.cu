@@ -112,8 +112,9 @@ StagedShape staged_shape(int nv, int groups) {
 }
 
 // Dynamic shared memory: the ring's mbarriers and counts, the stages' columns, the sums of
-// the candidate groups, the stages' entries, the line tables (sized for the largest item of
-// a launch, laid out per item from the launch's own strides).
+// the candidate groups, the stages' entries, the line tables.  Laid out for the largest volume
+// and the longest columns of a launch: while the producers fill the next item's stages, the
+// consumers still read the last one's.
 constexpr int kRing = 3, kProducers = 3;
 // A producer that filled stage i knows stage i - kRing consumed; the parity it waits for
 // before stage i + kProducers tells that stage's slot one phase back from two only if the
@@ -457,7 +458,7 @@ __device__ __forceinline__ bool staged_produce(const StagedItem &I, const Staged
             if (out_stage >= 0) mbar_wait(&ring->full[out_stage], out_parity);
             break;
         }
-        float *dst = columns + ((size_t)my.stage * L.slots + __popc(all & below)) * xst;
+        float *dst = columns + ((size_t)my.stage * L.slots + __popc(all & below)) * L.xstride;
         const uint32_t xadj = smem_addr(dst) - (0x4B000000u << 2);
 #pragma unroll
         for (int h = 0; h < 4; h++)
@@ -604,8 +605,10 @@ struct StagedRegs {
     static_assert(128 * (kProducer + CW * kConsumer) <= 128 * (1 + CW) * kLaunch || NP <= 2, "register split");
 };
 
+// xstride: the columns' stride in the stages, the same for all items (0: the only plan's own).
 template <int METHOD, int NP, int CW, int TAPS, class ITEM>
-__device__ __forceinline__ void staged_block(int total, int groups, int parts, int slots, int nlines, ITEM item) {
+__device__ __forceinline__ void staged_block(int total, int groups, int parts, int slots, int xstride, int nlines,
+                                             ITEM item) {
     extern __shared__ float4 smem_staged[];
     StagedRing *ring = reinterpret_cast<StagedRing *>(smem_staged);
     constexpr int consumers = 128 * CW;
@@ -627,14 +630,14 @@ __device__ __forceinline__ void staged_block(int total, int groups, int parts, i
         if (threadIdx.x >= 32 * kProducers) return;
         for (int blk = blockIdx.x; blk < total; blk += gridDim.x) {
             const StagedItem I = item(blk);
-            L.xstride = I.g->xstride;
+            L.xstride = xstride ? xstride : I.g->xstride;
             if (!staged_produce<METHOD>(I, L, ring, at, wg * NP)) return;
         }
     } else {
         if constexpr (NP > 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(StagedRegs<NP, CW>::kConsumer));
         for (int blk = blockIdx.x; blk < total; blk += gridDim.x) {
             const StagedItem I = item(blk);
-            L.xstride = I.g->xstride;
+            L.xstride = xstride ? xstride : I.g->xstride;
             if (!staged_consume<NP, TAPS>(I, L, ring, at, wg, consumers)) return;
         }
     }
@@ -647,7 +650,7 @@ __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * Stag
                        const uint8_t *__restrict__ state, void *__restrict__ proj,
                        int out_dtype, int view_begin, int view_stride, float margin, int groups, int parts,
                        int slots, int *__restrict__ err, int ngx, int vc, int total) {
-    staged_block<METHOD, NP, CW, TAPS>(total, groups, parts, slots, max(g.nx, g.ny), [&](int blk) {
+    staged_block<METHOD, NP, CW, TAPS>(total, groups, parts, slots, 0, max(g.nx, g.ny), [&](int blk) {
         StagedItem I{&g, views, xs, ampv, state, proj, err, out_dtype, view_begin, view_stride, 0, 0, 0, margin};
         const int per = ngx * vc;
         I.bz = blk / per;
@@ -656,13 +659,14 @@ __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * Stag
     });
 }
 
-// The staged forward projector over the items of many plans (same launch shape, slots and
-// column stride; each task its own geometry, scratch and storage type).  nlines: the
-// largest volume's.
+// The staged forward projector over the items of many plans of one launch shape and TAPS (each
+// task its own geometry, scratch and storage type).  xstride, nlines: the longest columns' and
+// the largest volume's.
 template <int METHOD, int NP, int CW, int TAPS>
 __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * StagedRegs<NP, CW>::kLaunch))
-    proj_staged_batch_kernel(const __grid_constant__ ProjBatch b, int groups, int parts, int slots, int nlines) {
-    staged_block<METHOD, NP, CW, TAPS>(b.total, groups, parts, slots, nlines, [&](int blk) {
+    proj_staged_batch_kernel(const __grid_constant__ ProjBatch b, int groups, int parts, int slots, int xstride,
+                             int nlines) {
+    staged_block<METHOD, NP, CW, TAPS>(b.total, groups, parts, slots, xstride, nlines, [&](int blk) {
         int lo = 0, hi = b.n - 1;
         while (lo < hi) {
             const int m = (lo + hi + 1) >> 1;
@@ -682,10 +686,12 @@ __global__ void __launch_bounds__(128 * (1 + CW), 65536 / (128 * (1 + CW) * Stag
 // ---------------------------------------------------------------------------
 // Work items along the detector columns.
 int staged_columns(const StagedShape &S, int nu) { return (nu + kPart * S.parts - 1) / (kPart * S.parts); }
-size_t proj_staged_smem_bytes(int nv, int nlines, int xstride, int groups, int slots) {
-    const StagedShape S = staged_shape(nv, groups);
+size_t proj_staged_smem_bytes(const StagedShape &S, int nlines, int xstride, int slots) {
     StagedSmem L{nlines, slots, xstride, S.warps * S.np, S.groups, S.parts};
     return L.bytes();
+}
+size_t proj_staged_smem_bytes(int nv, int nlines, int xstride, int groups, int slots) {
+    return proj_staged_smem_bytes(staged_shape(nv, groups), nlines, xstride, slots);
 }
 // Slots per stage: 1 .. 64 (at most 32 are used), and their bytes within an mbarrier phase's
 // transaction count (< 2^20).
@@ -732,11 +738,11 @@ cudaError_t launch_proj_staged(int method, int groups, int slots, const ColumnsG
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_proj_staged_batch(int method, const StagedShape &S, int taps, int slots, int nlines, size_t sm,
-                                     const ProjBatch &b, cudaStream_t st) {
+cudaError_t launch_proj_staged_batch(int method, const StagedShape &S, int taps, int slots, int xstride, int nlines,
+                                     size_t sm, const ProjBatch &b, cudaStream_t st) {
     if (b.n < 1 || b.total < 1) return cudaSuccess;
     CTSIM_STAGED_SWITCH(proj_staged_batch_kernel, (k<<<persistent_grid((const void *)k, nt, sm, b.total), nt, sm, st>>>(
-                                                      b, S.groups, S.parts, slots, nlines)));
+                                                      b, S.groups, S.parts, slots, xstride, nlines)));
     return cudaErrorInvalidValue;
 }
 
