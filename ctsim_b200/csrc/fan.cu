@@ -16,8 +16,8 @@
 // The footprints are chains of exactly rounded divisions and the sums are serial, so both are
 // bound by latency; what helps is to evaluate ahead of the sums, in parallel.  Measured on
 // B200, DD pair at 256^2, 360 bins, 180 views: 1.95 -> 0.81 ms (A 0.70, A^T 0.11) against one warp
-// per 32 bins and one thread per pixel, doing both in turn.  Results do not depend on the
-// launch.
+// per 32 bins and one thread per pixel, doing both in turn.  The former still serves the wide
+// footprints (fan_proj_warp_kernel, fan_wide).  Results do not depend on the launch.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -354,6 +354,133 @@ __global__ void __launch_bounds__(kFanThreads) fan_proj_kernel(FanGeom g, const 
     if (bin >= 0 && iu0 + bin < g.nu) proj[(size_t)k * g.nu + iu0 + bin] = (float)acc;
 }
 
+// Footprints of three bins and more: one warp per (32 bins, view), a candidate per lane, then
+// each candidate's bins in turn.  Many lanes add at once there, and nothing is evaluated twice.
+// Shared memory: per row the first candidate column and the running candidate count, then one
+// candidate record per lane.
+template <bool TF>
+__global__ void __launch_bounds__(32) fan_proj_warp_kernel(FanGeom g, const FanView *__restrict__ views,
+                                                      const float *__restrict__ image, float *__restrict__ proj,
+                                                      int view_begin, int view_stride) {
+    extern __shared__ int fsw[];
+    int *row_first = fsw;                      // [ny]
+    int *row_off = fsw + g.ny;                 // [ny + 1]
+    float *c_t = reinterpret_cast<float *>(row_off + g.ny + 1);  // [4][32]
+    float *c_amp = c_t + 4 * 32;               // [32]: DD amplitude, SF amplitude * pixel
+    float *c_x = c_amp + 32;                   // [32]: DD pixel value
+    int *c_lo = reinterpret_cast<int *>(c_x + 32);
+    int *c_hi = c_lo + 32;
+    const int lane = threadIdx.x;
+    const int iu0 = blockIdx.x * 32;
+    const int k = blockIdx.y;
+    const FanView v = views[view_begin + k * view_stride];
+    const float ulo = (float)iu0 - g.margin, uhi = (float)(iu0 + 32) + g.margin;
+    // approximate projected centre (candidate search only; footprints are exact below)
+    auto centre = [&](int ix, int iy) {
+        const float xc = ((float)ix + g.wx) * g.dx, yc = ((float)iy + g.wy) * g.dy;
+        const float r = (xc * v.cos_a - yc * v.sin_a) / (g.sad + xc * v.sin_a + yc * v.cos_a);
+        return (g.det == 1 ? g.sdd_du * r : g.sdd_du * atanf(r)) - g.wu + 0.5f;
+    };
+    for (int iy = lane; iy < g.ny; iy += 32) {
+        const bool inc = centre(g.nx - 1, iy) >= centre(0, iy);
+        int lo = 0, hi = g.nx;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            const float f = centre(mid, iy);
+            if (inc ? (f < ulo) : (f > uhi)) lo = mid + 1; else hi = mid;
+        }
+        const int first = lo;
+        hi = g.nx;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            const float f = centre(mid, iy);
+            if (inc ? (f > uhi) : (f < ulo)) hi = mid; else lo = mid + 1;
+        }
+        row_first[iy] = first;
+        row_off[iy] = lo - first;
+    }
+    __syncwarp();
+    {   // exclusive scan of the per-row counts (lane owns a contiguous run of rows)
+        const int per = (g.ny + 31) / 32;
+        const int b = min(lane * per, g.ny), e = min(b + per, g.ny);
+        int sum = 0;
+        for (int iy = b; iy < e; iy++) sum += row_off[iy];
+        int incl = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += n;
+        }
+        __syncwarp();
+        int run = incl - sum;
+        for (int iy = b; iy < e; iy++) {
+            const int c = row_off[iy];
+            row_off[iy] = run;
+            run += c;
+        }
+        if (lane == 31) row_off[g.ny] = incl;
+    }
+    __syncwarp();
+    const int ncand = row_off[g.ny];
+    const int iu = iu0 + lane;
+    float acc = 0.0f;
+    for (int c0 = 0; c0 < ncand; c0 += 32) {
+        const int c = c0 + lane;
+        int lo = 0, hi = -1;
+        if (c < ncand) {
+            int a = 0, z = g.ny - 1;  // last row with row_off <= c
+            while (a < z) {
+                const int mid = (a + z + 1) >> 1;
+                if (row_off[mid] <= c) a = mid; else z = mid - 1;
+            }
+            const int iy = a, ix = row_first[a] + (c - row_off[a]);
+            float t[4];
+            const float amp = fan_pixel<TF>(g, v, ix, iy, t);
+            float umin, umax;
+            if (fan_range(g, t[0], TF ? t[3] : t[1], umin, umax, lo, hi)) {
+                const float x = image[(size_t)iy * g.nx + ix];
+                if (TF) {
+                    for (int q = 0; q < 4; q++) c_t[q * 32 + lane] = t[q];
+                    c_amp[lane] = fmul(amp, x);  // voxel = amplitude * image
+                } else {
+                    c_t[lane] = umin;
+                    c_t[32 + lane] = umax;
+                    c_amp[lane] = amp;
+                    c_x[lane] = x;
+                }
+            } else {
+                lo = 0;
+                hi = -1;
+            }
+        }
+        c_lo[lane] = lo;
+        c_hi[lane] = hi;
+        __syncwarp();
+        const int ns = min(32, ncand - c0);
+        for (int s = 0; s < ns; s++) {
+            const int slo = c_lo[s], shi = c_hi[s];
+            if (iu < slo || iu > shi) continue;
+            if (TF) {
+                float t[4] = {c_t[s], c_t[32 + s], c_t[64 + s], c_t[96 + s]};
+                acc = fadd(acc, fmul(fan_tf_weight(iu, t), c_amp[s]));
+            } else {
+                const float umin = c_t[s], umax = c_t[32 + s], amp = c_amp[s], x = c_x[s];
+                if (slo == shi) {
+                    acc = fadd(acc, fmul(fmul(amp, fsub(umax, umin)), x));
+                } else if (iu == slo) {  // amplitude * (iumin + 1.0 - umin) * image, in double
+                    const double w = __dsub_rn(__dadd_rn((double)slo, 1.0), (double)umin);
+                    acc = (float)__dadd_rn((double)acc, __dmul_rn(__dmul_rn((double)amp, w), (double)x));
+                } else if (iu == shi) {
+                    acc = fadd(acc, fmul(fmul(amp, fsub(umax, (float)shi)), x));
+                } else {
+                    acc = fadd(acc, fmul(amp, x));
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (iu < g.nu) proj[(size_t)k * g.nu + iu] = acc;
+}
+
 // One pixel in one view: what the view adds to the pixel (0 where it has no bin).
 template <bool TF>
 __device__ __forceinline__ float fan_back_view(const FanGeom &g, const FanView &v, const float *__restrict__ p, int ix,
@@ -431,6 +558,29 @@ struct ctsim_fan_plan {
 };
 
 static size_t fan_proj_smem(int ny) { return 2 * sizeof(FanStep) + (size_t)(2 * ny + 1) * 4; }
+static size_t fan_proj_warp_smem(int ny) { return (size_t)(2 * ny + 1) * 4 + 32 * 6 * 4 + 32 * 2 * 4; }
+
+// Whether A takes a warp per 32 bins: footprints so wide (in bins, nearest the source; SF's at 45
+// degrees) that some touch more bins than a step keeps contributions of and would be evaluated
+// again for each.  DD, pixels of 2.5, 2.7 and 3 bins (3.1, 3.4 and 3.8 at the nearest), 90 views, steps
+// over warps: 64^2 0.58, 1.75, 2.06, 256^2 0.57, 2.00, 3.39, 512^2 0.68, 1.49, 2.34; SF, pixels of 2, 2.04
+// and 2.5 bins (3.6, 3.7 and 4.5): 64^2 0.35, 0.37, 1.21, 256^2 0.35, 0.37, 0.67, 512^2 0.42, 0.38, 0.80, on
+// curved detectors 0.49, 0.54, 1.79; 0.35, 0.38, 0.97; 0.44, 0.41, 1.12.
+constexpr float kFanWideDD = 3.25f, kFanWideTF = 3.75f;
+static bool fan_wide(const ctsim_fan_plan *p, int method) {
+    const ctsim_fan_geom &G = p->geom;
+    if (method != CTSIM_PROJ_DD) return 2.0f * p->g.reach >= kFanWideTF;
+    return 2.0f * p->g.reach * std::max(G.dx, G.dy) / std::hypot(G.dx, G.dy) >= kFanWideDD;
+}
+
+// A kernel with its dynamic shared memory; the launch's error.
+template <class K, class... Args>
+static cudaError_t fan_launch(K kernel, dim3 grid, int threads, size_t smem, void *stream, Args... args) {
+    cudaError_t e = allow_dynamic_smem((const void *)kernel, smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, threads, smem, (cudaStream_t)stream>>>(args...);
+    return cudaGetLastError();
+}
 
 extern "C" ctsim_status ctsim_fan_plan_create(const ctsim_fan_geom *geom, const double *betas, ctsim_fan_plan **out) {
     if (!geom || !betas || !out) return ctsim_set_last_error(CTSIM_ERR_ARGUMENT, "null argument");
@@ -515,21 +665,16 @@ extern "C" ctsim_status ctsim_fan_project(ctsim_fan_plan *p, int method, const f
         return ctsim_set_last_error(CTSIM_ERR_ARGUMENT, "unknown forward method");
     ctsim_status s = fan_views_ok(p, view_begin, view_stride, view_count);
     if (s != CTSIM_OK) return s;
-    const size_t sm = fan_proj_smem(p->g.ny);
-    dim3 grid((p->g.nu + kFanBins - 1) / kFanBins, view_count);
+    const bool dd = method == CTSIM_PROJ_DD;
     cudaError_t e;
-    if (method == CTSIM_PROJ_DD) {
-        if ((e = allow_dynamic_smem((const void *)fan_proj_kernel<false>, sm)) != cudaSuccess)
-            return ctsim_set_last_error(CTSIM_ERR_CUDA, cudaGetErrorString(e));
-        fan_proj_kernel<false><<<grid, kFanThreads, sm, (cudaStream_t)stream>>>(p->g, p->d_views, d_image, d_sino, view_begin,
-                                                                       view_stride);
-    } else {
-        if ((e = allow_dynamic_smem((const void *)fan_proj_kernel<true>, sm)) != cudaSuccess)
-            return ctsim_set_last_error(CTSIM_ERR_CUDA, cudaGetErrorString(e));
-        fan_proj_kernel<true><<<grid, kFanThreads, sm, (cudaStream_t)stream>>>(p->g, p->d_views, d_image, d_sino, view_begin,
-                                                                      view_stride);
-    }
-    e = cudaGetLastError();
+    if (fan_wide(p, method))
+        e = fan_launch(dd ? fan_proj_warp_kernel<false> : fan_proj_warp_kernel<true>, dim3((p->g.nu + 31) / 32, view_count),
+                       32, fan_proj_warp_smem(p->g.ny), stream, p->g, p->d_views, d_image, d_sino, view_begin,
+                       view_stride);
+    else
+        e = fan_launch(dd ? fan_proj_kernel<false> : fan_proj_kernel<true>,
+                       dim3((p->g.nu + kFanBins - 1) / kFanBins, view_count), kFanThreads, fan_proj_smem(p->g.ny), stream,
+                       p->g, p->d_views, d_image, d_sino, view_begin, view_stride);
     return e == cudaSuccess ? CTSIM_OK : ctsim_set_last_error(CTSIM_ERR_CUDA, cudaGetErrorString(e));
 }
 
@@ -541,14 +686,14 @@ extern "C" ctsim_status ctsim_fan_backproject(ctsim_fan_plan *p, int method, con
         return ctsim_set_last_error(CTSIM_ERR_ARGUMENT, "unknown fan-beam backprojection method");
     ctsim_status s = fan_views_ok(p, view_begin, view_stride, view_count);
     if (s != CTSIM_OK) return s;
-    dim3 grid((p->g.nx + 31) / 32, p->g.ny);
+    const dim3 grid((p->g.nx + 31) / 32, p->g.ny);
     if (method == CTSIM_BACK_DD)
         fan_back_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(p->g, p->d_views, d_sino, d_image, view_begin,
                                                                        view_stride, view_count, scale);
     else
         fan_back_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(p->g, p->d_views, d_sino, d_image, view_begin,
                                                                       view_stride, view_count, scale);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CTSIM_OK : ctsim_set_last_error(CTSIM_ERR_CUDA, cudaGetErrorString(e));
 }
 
