@@ -16,8 +16,9 @@
 // The footprints are chains of exactly rounded divisions and the sums are serial, so both are
 // bound by latency; what helps is to evaluate ahead of the sums, in parallel.  Measured on
 // B200, DD pair at 256^2, 360 bins, 180 views: 1.95 -> 0.81 ms (A 0.70, A^T 0.11) against one warp
-// per 32 bins and one thread per pixel, doing both in turn.  The former still serves the wide
-// footprints (fan_proj_warp_kernel, fan_wide).  Results do not depend on the launch.
+// per 32 bins and one thread per pixel, doing both in turn.  Those still serve the wide footprints
+// (fan_proj_warp_kernel), the few views and the large images (fan_back_pixel_kernel) for which
+// they are the faster ones (fan_wide, fan_back_by_pixel).  Results do not depend on the launch.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -548,6 +549,22 @@ __global__ void __launch_bounds__(256) fan_back_kernel(FanGeom g, const FanView 
     }
 }
 
+// One thread per pixel, the views in order.
+template <bool TF>
+__global__ void __launch_bounds__(128) fan_back_pixel_kernel(FanGeom g, const FanView *__restrict__ views,
+                                                             const float *__restrict__ proj, float *__restrict__ image,
+                                                             int view_begin, int view_stride, int view_count,
+                                                             float scale) {
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y;
+    if (ix >= g.nx) return;
+    float img = 0.0f;
+    for (int k = 0; k < view_count; k++)
+        img = fadd(img, fan_back_view<TF>(g, views[view_begin + k * view_stride], proj + (size_t)k * g.nu, ix, iy));
+    if (scale != 1.0f) img = img * scale;
+    image[(size_t)iy * g.nx + ix] = img;
+}
+
 }  // namespace
 
 struct ctsim_fan_plan {
@@ -571,6 +588,15 @@ static bool fan_wide(const ctsim_fan_plan *p, int method) {
     const ctsim_fan_geom &G = p->geom;
     if (method != CTSIM_PROJ_DD) return 2.0f * p->g.reach >= kFanWideTF;
     return 2.0f * p->g.reach * std::max(G.dx, G.dy) / std::hypot(G.dx, G.dy) >= kFanWideDD;
+}
+
+// Whether A^T takes a thread per pixel: where the image alone fills the GPU, or the views leave
+// most of a block's warps without one.  Block kernel over pixel kernel, DD, flat: 1, 8, 16, 32 and
+// 64 views at 64^2 0.86, 0.75, 0.46, 0.27, 0.21; 256^2 1.45, 1.29, 0.95, 0.69, 0.62; 512^2 2.59, 1.83,
+// 1.25, 0.94, 0.91; 1024^2 4.51, 2.12, 1.31, 1.02, 0.99; 2000^2 5.79, 2.20, 1.34, 1.04, 1.01.
+static bool fan_back_by_pixel(const ctsim_fan_geom &G, int view_count) {
+    const long long pixels = (long long)G.nx * G.ny;
+    return view_count < 8 || pixels >= (view_count < 16 ? 1 << 15 : view_count < 32 ? 1 << 18 : 1 << 20);
 }
 
 // A kernel with its dynamic shared memory; the launch's error.
@@ -686,13 +712,13 @@ extern "C" ctsim_status ctsim_fan_backproject(ctsim_fan_plan *p, int method, con
         return ctsim_set_last_error(CTSIM_ERR_ARGUMENT, "unknown fan-beam backprojection method");
     ctsim_status s = fan_views_ok(p, view_begin, view_stride, view_count);
     if (s != CTSIM_OK) return s;
-    const dim3 grid((p->g.nx + 31) / 32, p->g.ny);
-    if (method == CTSIM_BACK_DD)
-        fan_back_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(p->g, p->d_views, d_sino, d_image, view_begin,
-                                                                       view_stride, view_count, scale);
-    else
-        fan_back_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(p->g, p->d_views, d_sino, d_image, view_begin,
-                                                                      view_stride, view_count, scale);
+    const bool dd = method == CTSIM_BACK_DD;
+    const bool pixel = fan_back_by_pixel(p->geom, view_count);
+    const dim3 grid((p->g.nx + (pixel ? 127 : 31)) / (pixel ? 128 : 32), p->g.ny);
+    const auto kernel = pixel ? (dd ? fan_back_pixel_kernel<false> : fan_back_pixel_kernel<true>)
+                              : (dd ? fan_back_kernel<false> : fan_back_kernel<true>);
+    kernel<<<grid, pixel ? 128 : 256, 0, (cudaStream_t)stream>>>(p->g, p->d_views, d_sino, d_image, view_begin, view_stride,
+                                                                 view_count, scale);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CTSIM_OK : ctsim_set_last_error(CTSIM_ERR_CUDA, cudaGetErrorString(e));
 }

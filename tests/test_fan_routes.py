@@ -1,5 +1,5 @@
-"""The 2-D projector on both sides of the line between its kernels (footprints of a few bins or
-many) and candidate counts at the edges of a step of 192.
+"""The 2-D pair on both sides of the lines between its kernels -- footprints of a few bins or many,
+few views or many, small images or large -- and candidate counts at the edges of a step of 192.
 Bit-identical to the reference restatement on flat detectors."""
 import numpy as np
 import pytest
@@ -47,3 +47,19 @@ def test_projection_at_a_steps_edges(size):
     for m in ("dd", "tf"):
         got = plan.project(torch.from_numpy(x).cuda(), m).cpu().numpy()
         assert np.array_equal(got, oracle_fbct(f"proj,{m}", g, x)), m
+
+
+@pytest.mark.parametrize("size,views", [((20, 9), (1, 7, 8, 33)), ((200, 163), (7, 8, 15, 16)), ((200, 164), (8, 15, 16)),
+                                        ((512, 512), (15, 16, 31, 32)), ((1030, 1020), (32, 40))])
+def test_backprojection_across_views_and_sizes(size, views):
+    import torch
+    from ctsim_b200.fan import FanPlan
+    from oracle.bindings import oracle_fbct
+    nx, ny = size
+    for v in views:
+        g = _geom(nx, ny, 100.0 / nx, 70, 2.5, circular_betas(v) + 0.02)
+        y = np.random.default_rng(v).random(g.sino_shape, dtype=np.float32)
+        plan = FanPlan(g)
+        for m in ("dd", "tf"):
+            got = plan.backproject(torch.from_numpy(y).cuda(), m, scale=2.0).cpu().numpy()
+            assert np.array_equal(got, np.float32(2.0) * oracle_fbct(f"back,{m}", g, y)), (v, m)
