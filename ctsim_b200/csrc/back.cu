@@ -346,10 +346,12 @@ __device__ __forceinline__ void back_block(const Geom &g, const View *__restrict
     }
 }
 
-// Four resident blocks per SM (registers capped at 64): measured on B200 at config 2,
-// DD 110 -> 100 ms and SF 143 -> 104 ms against the uncapped 80-118 registers.
+// Four resident blocks per SM (registers capped at 64): measured on B200 at 512^2 x 256 and 720
+// views, DD 110 -> 100 ms and SF 143 -> 104 ms against the uncapped 80-118 registers.  The geometry
+// stays in the parameters: copied, its size decides which values spill (128^2 x 64, BF16, 360 views
+// 0.995 -> 1.013 ms).
 template <int METHOD, int MZ, bool VEC, int SRC = kSrcScaled, bool SUM = false>
-__global__ void __launch_bounds__(256, 4) back_kernel(Geom g, const View *__restrict__ views,
+__global__ void __launch_bounds__(256, 4) back_kernel(const __grid_constant__ Geom g, const View *__restrict__ views,
                                                    const void *__restrict__ ps, const uint8_t *__restrict__ map,
                                                    void *__restrict__ image, int out_dtype, int view_begin,
                                                    int view_stride, int view_count, float scale, int qcap,
