@@ -300,7 +300,8 @@ __device__ __forceinline__ void back_block(const Geom &g, const View *__restrict
                         const uint32_t qrow = qadj + (0x4B000000u << 2);
                         auto qb = [&](int k) { return lds_ordered(qrow + 4u * (uint32_t)k); };
 #pragma unroll
-                        for (int p = 0; p < NP; p++)
+                        for (int p = 0; p < NP; p++) {
+                            if (p > 0 && 32 * W * p >= izn) break;  // warp-uniform
                             acc[p] = P::make([&](int i) {
                                 const float izv = P::get(fz[p], i);
                                 const float vpre = fadd(pa.z, fmul(izv, pa.y));
@@ -324,11 +325,13 @@ __device__ __forceinline__ void back_block(const Geom &g, const View *__restrict
                                     vox = fsub(vmax, vmin) * qb(klo);
                                 } else if (klo < khi) {
                                     vox = fsub(fadd(flo, 1.0f), vmin) * qb(klo);
+                                    #pragma unroll 4
                                     for (int k = klo + 1; k < khi; k++) vox += qb(k);
                                     vox = fmaf(fsub(vmax, fhi), qb(khi), vox);
                                 }
                                 return fmaf(pa.x, vox, a);
                             });
+                        }
                     }
                     __syncwarp();
                 }

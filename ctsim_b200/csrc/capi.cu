@@ -389,7 +389,12 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
         int mz = std::min(8, pow2_at_least((G.nz + 31) / 32));
         while (mz > 1 && !back_mz_fits(p, mz)) mz >>= 1;
         p->back_mz = p->back_mz_tf = mz;
-        p->back_qcap = p->back_qcap_tf = back_qcap_for(p, mz);
+        // SF, voxels of more than two rows (the loop of back.cu): the pass of eight blocks spills more
+        // than it saves.  Voxels of 2.5 and 5 rows, passes of four and eight blocks: 200^2 x 160, 60
+        // views 2.09, 3.14 and 2.33, 3.52 ms; 300^2 x 300, 24 views 3.19, 4.89 and 3.94, 7.88 ms.
+        if ((double)G.dz / G.dv * G.sdd / G.sad > 2.0) p->back_mz_tf = std::min(mz, 4);
+        p->back_qcap = back_qcap_for(p, mz);
+        p->back_qcap_tf = back_qcap_for(p, p->back_mz_tf);
         // FDK: a pass of all slices up to 256, in pairs of 32-voxel blocks.  Measured on B200,
         // back,hpd with 1, 2, 4 and 8 blocks: 512^2 x 256, 90 views 11.6, 7.7, 7.4 and 7.1 ms;
         // 128^2 x 64, 360 views 0.79, 0.53, 0.60 and 0.60 ms (the longer kernels hold more
