@@ -199,8 +199,12 @@ __device__ __forceinline__ void pd_pass_of(int np, const Geom &g, const PdArgs &
     pd_pass<MODE, NP, V, DT>(g, A, vtab, ix, iy, iz0, on);
 }
 
+// Blocks per SM: four of the packed kernels (registers capped at 64); six of the scalar one, whose
+// loads only other warps hide (back,hpd of 512^2 x 32, 720 views of 72 rows: 13.5 ms with five, 10.9
+// with six; pd, 40 rows 11.6 and 10.8 ms).  The geometry stays in the parameters (a copy's size
+// decides how the kernel compiles: back,hpd of 128^2 x 64, 360 views 0.54 -> 0.60 ms).
 template <int MODE, int MZ, class V, int DT>
-__global__ void __launch_bounds__(256, MZ == 1 ? 5 : 4) pd_kernel(Geom g, PdArgs A, const uint8_t *__restrict__ map) {
+__global__ void __launch_bounds__(256, MZ == 1 ? 6 : 4) pd_kernel(const __grid_constant__ Geom g, PdArgs A, const uint8_t *__restrict__ map) {
     constexpr int W = Packed<V>::kWidth, NP = MZ / W;
     const int warp = threadIdx.x >> 5;
     const int tiles_x = (g.nx + 7) >> 3;
