@@ -11,6 +11,7 @@
 
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 namespace ctsim {
@@ -471,12 +472,23 @@ __global__ void __launch_bounds__(kProjMaxThreads) proj_batch_kernel(const __gri
 
 int proj_row_threads_of(int nv) { return proj_row_threads(nv); }
 
+// The resident blocks of a kernel's launch shape are asked for once per device: the staged forward
+// projector needs them at every launch, twelve times per OS-SQS iteration of twelve subsets.
 int persistent_grid(const void *kernel, int threads, size_t smem, int total) {
-    int dev = 0, sms = 148, per_sm = 1;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    return std::max(1, std::min(total, sms * per_sm));
+    static std::mutex m;
+    static std::map<std::tuple<int, const void *, int, size_t>, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+    std::lock_guard<std::mutex> lock(m);
+    int &resident = known[{dev, kernel, threads, smem}];
+    if (resident == 0) {
+        int sms = 148, per_sm = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
+            per_sm = 1;
+        resident = sms * per_sm;
+    }
+    return std::max(1, std::min(total, resident));
 }
 
 cudaError_t launch_proj_batch(int method, int groups, int row_threads, bool pairs, bool lowp, size_t smem,
