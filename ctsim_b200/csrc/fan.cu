@@ -127,7 +127,8 @@ constexpr int kFanThreads = kFanChunk + kFanBins;
 constexpr int kFanVals = 4;                       // bins of a footprint whose contributions are kept
 // Bins per pixel step along a row below which a bin gathers its pixels itself: at 256^2, 360
 // bins, one view 80 degrees off takes 0.30 ms in steps and 0.44 ms gathered, 84 degrees 0.73 and
-// 0.46 ms; all 180 views 0.90, 0.70 and 0.71 ms with the line at 0.1, 0.2 and 0.4.
+// 0.46 ms; all 180 views 0.88, 0.68 and 0.73 ms with the line at 0.1, 0.2 and 0.4; 128^2, 180 bins 0.36, 0.27 and
+// 0.29; 512^2, 720 bins 2.79, 1.79 and 2.07, 360 bins 1.71, 1.84 and 2.13; 256^2, 100 bins 0.77, 0.76 and 0.93.
 constexpr float kFanGatherBelow = 0.2f;
 constexpr int kFanLanes = kFanThreads / kFanBins; // lanes per bin of the gather
 static_assert(kFanLanes == 4, "one bin per four lanes");

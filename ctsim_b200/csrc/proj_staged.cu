@@ -30,11 +30,12 @@
 //
 // What bounds it: instruction issue (58% of the slots) and the waits at the stages' ends.
 // Measured on B200 against row threads that kept their sums in shared memory and read prefix
-// sums: DD A of 512^2 x 256 and 720 views of 1024 x 384 106.4 -> 63.3 ms; against the
+// sums: DD A of 512^2 x 256 and 720 views of 1024 x 384 106.4 -> 63.4 ms; against the
 // unstaged projector over paired prefix sums, 128^2 x 64 and 360 views of 256 x 96 2.08 ->
-// 0.90 ms.  On the way, 96 of the 720 views: one producer 14.0 ms, four on a ring of four 9.6,
-// packed arithmetic through the float2 intrinsics instead of inline assembly (fewer moves)
-// 9.2.
+// 0.91 ms.  On the way, 96 of the 720 views: one producer 14.0 ms, four on a ring of four 9.6,
+// packed arithmetic through the float2 intrinsics instead of inline assembly (fewer moves) 9.2.
+// Rows of more than three voxels on large volumes, and columns too tall for three stages, take
+// proj_sums.cu.
 #include <algorithm>
 #include <cmath>
 

@@ -342,9 +342,10 @@ def batched_subset_steps(pairs):
 class BatchedPwls:
     """Many OS-PWLS reconstructions (reconPwlsSeSqs.m:57-66 each) stepped together.
 
-    Every sub-iteration runs ONE persistent A launch over all instances' subset views
-    (ctsim_batch_project, per launch-shape class), the per-instance residuals, ONE
-    persistent A^T launch (ctsim_batch_backproject) and the per-instance SQS updates;
+    Every sub-iteration runs one persistent A launch over all instances' subset views
+    (ctsim_batch_project; one per launch-shape class, which plans of different slices
+    share), the per-instance residuals, one persistent A^T launch likewise
+    (ctsim_batch_backproject) and the per-instance SQS updates;
     with ``graphs`` an outer iteration of all instances is one CUDA-graph replay after
     the first.  The instances keep their own plans, data and state, so each result is
     the one its own solver would compute.  All solvers use the same projector method

@@ -184,26 +184,31 @@ ctsim_status ctsim_plan_create_async(const ctsim_geom *geom, const double *betas
 ctsim_status ctsim_pool_trim(size_t keep_bytes);
 
 /* Launch shapes of a plan (no reference counterpart): the forward projector's
- * candidate-parallel groups (1, 2, 4, 8; layout 3 uses at most four) and the 32-voxel z blocks per lane of
- * the A^T passes (back_mz for DD, back_mz_tf for SF) and of the FDK/var kernel (pd_mz),
- * each 1, 2, 4 or 8.  Plans start with a size rule; set_tuning changes the non-zero
- * fields (validated against the geometry).  The group count and the A^T z blocks change
- * the floating-point rounding of A and A^T (the summation order and the start of the
- * running row sums), never the footprints; the FDK/var z blocks change nothing. */
+ * candidate-parallel groups (1, 2, 4, 8; voxel columns use at most four) and the 32-voxel z
+ * blocks per lane of the A^T passes (back_mz for DD, back_mz_tf for SF) and of the FDK/var kernel
+ * (pd_mz), each 1, 2, 4 or 8.  Plans start with a size rule; set_tuning changes the non-zero
+ * fields (validated against the geometry and the layout that results).  The group count is
+ * that of the layout's projector: voxel columns have one of their own, the other forms share
+ * one.  It changes the floating-point rounding of A (the summation order), never the
+ * footprints; the z blocks change no result. */
 typedef struct {
     int proj_groups;
     int back_mz;
     int pd_mz;
     int back_mz_tf;
-    int proj_rows;  /* layouts 1 and 2: row threads per forward group, a multiple of 32 up to
+    int proj_rows;  /* row threads per forward group (not of voxel columns), a multiple of 32 up to
                        ceil(nv/4) rounded to whole warps; 32 makes each group one warp that walks
                        only the rows of each candidate's shadow */
     int proj_layout; /* the image's form: 1 column prefix sums, 2 (sum, slope) pairs (one 8-byte load
                         per evaluation; twice the bytes; plans whose pairs take at most 160 MB may
-                        switch to it), 3 voxel columns, each candidate's copied into shared memory by
-                        the copy engine (what plans start with where a detector row reaches at most
-                        three voxels, and where pairs are not available) */
-    int proj_slots;  /* layout 3: columns per stage, 1 .. 64 (at most 32 are used) */
+                        switch to it), 3 columns copied into shared memory by the copy engine, each
+                        candidate's whole: voxel columns where a detector row reaches at most three
+                        voxels, or at most eight on columns of up to 256 slices (128 where pairs take
+                        more than 160 MB), as far as three stages of eight fit; prefix sums elsewhere.
+                        Plans start with voxel columns, else with pairs, else with staged sums, else
+                        (columns of which two stages of eight do not fit) with 1 */
+    int proj_slots;  /* layout 3: columns per stage, 1 .. 64 (of voxel columns at most 32, and as many as
+                        three stages of fit, are used) */
 } ctsim_tuning;
 ctsim_status ctsim_plan_get_tuning(const ctsim_plan *plan, ctsim_tuning *tuning);
 ctsim_status ctsim_plan_set_tuning(ctsim_plan *plan, const ctsim_tuning *tuning);
