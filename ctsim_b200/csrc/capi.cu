@@ -65,7 +65,7 @@ struct ctsim_plan {
     float *d_ampv = nullptr;
     uint8_t *d_map = nullptr;
     float *d_xs = nullptr;   // voxel columns or their prefix sums [nx*ny][g.xstride] (or pairs [nx*ny][nz+1][2]) -- forward scratch
-    uint8_t *d_xstate = nullptr;  // per voxel column: its map entry and whether its voxels are finite (staged projector)
+    uint8_t *d_xstate = nullptr;  // per staged voxel column: its map entry and whether it is finite; in d_xs's allocation
     float *d_ps = nullptr;   // sinogram scaled by ampv [noviews][nu][nv] -- backprojector scratch
     int *d_err = nullptr;
     size_t bytes = 0;
@@ -154,7 +154,6 @@ static void free_plan(ctsim_plan *p) {
     ctsim_plan_release(p, p->d_ampv);
     ctsim_plan_release(p, p->d_map);
     ctsim_plan_release(p, p->d_xs);
-    ctsim_plan_release(p, p->d_xstate);
     ctsim_plan_release(p, p->d_ps);
     ctsim_plan_release(p, p->d_err);
     delete p;
@@ -429,9 +428,9 @@ static ctsim_status create_plan(const ctsim_geom *geom, const double *betas, con
     p->fwd_staged = p->fwd_columns || (!p->xs_holds_pairs && staged_fits(p, p->fwd_slots));
     p->fwd_pairs = p->xs_holds_pairs && !p->fwd_staged;
     if (p->fwd_ok) {
-        CTSIM_ALLOC(p->d_xs, sizeof(float) * (size_t)nxy *
-                                 std::max(g.xstride, p->xs_holds_pairs ? 2 * (G.nz + 1) : 0));
-        CTSIM_ALLOC(p->d_xstate, (size_t)nxy);
+        const size_t floats = (size_t)nxy * std::max(g.xstride, p->xs_holds_pairs ? 2 * (G.nz + 1) : 0);
+        CTSIM_ALLOC(p->d_xs, sizeof(float) * floats + (p->fwd_columns ? (size_t)nxy : 0));
+        if (p->fwd_columns) p->d_xstate = reinterpret_cast<uint8_t *>(p->d_xs + floats);
     }
     // the backprojection scratch (an FP32 copy of the sinogram times ampv) is allocated on
     // first use (ensure_scratch): BF16/FP16 sinograms and CTSIM_INPUT_SCALED residuals are
